@@ -54,11 +54,11 @@ struct n2w_batch {
 namespace n2w {
 namespace {
 
-__global__ void rebase_nodes_kernel(const Node4* __restrict__ src, int64_t n, Node4* __restrict__ dst,
+__global__ void rebase_nodes_kernel(const FrameNode4* __restrict__ src, int64_t n, FrameNode4* __restrict__ dst,
                                     int32_t node_off, int32_t tri_off) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  Node4 nd = src[i];
+  FrameNode4 nd = src[i];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const int32_t r = nd.child[c];
@@ -211,7 +211,7 @@ int n2w_scene_create(const n2w_bvh* const* bvhs, int count, n2w_scene** out) {
     sc->meshes.resize(count);
     for (int k = 0; k < count; ++k) {
       const n2w_bvh* b = bvhs[k];
-      N2W_REQUIRE(b && b->d_nodes && b->d_tris, "n2w_scene_create: null BVH");
+      N2W_REQUIRE(b && b->d_frames && b->d_tris, "n2w_scene_create: null BVH");
       N2W_REQUIRE(b->device == sc->device, "n2w_scene_create: BVH on another device");
       auto& m = sc->meshes[k];
       m.node_off = sc->nodes;
@@ -235,13 +235,13 @@ int n2w_scene_create(const n2w_bvh* const* bvhs, int count, n2w_scene** out) {
     }
     N2W_REQUIRE(sc->nodes < (int64_t{1} << 31) && sc->tris < (int64_t{1} << 28),
                 "n2w_scene_create: merged scene exceeds 2^31 nodes or 2^28 triangles");
-    N2W_CUDA(cudaMalloc(&sc->d_nodes, sizeof(Node4) * sc->nodes));
+    N2W_CUDA(cudaMalloc(&sc->d_nodes, sizeof(FrameNode4) * sc->nodes));
     N2W_CUDA(cudaMalloc(&sc->d_tris, sizeof(TriRec) * sc->tris));
     if (sc->slots) N2W_CUDA(cudaMalloc(&sc->d_slots, sizeof(int) * sc->slots));
     for (int k = 0; k < count; ++k) {
       const n2w_bvh* b = bvhs[k];
       const auto& m = sc->meshes[k];
-      rebase_nodes_kernel<<<blocks_of(b->stats.nodes, 256), 256>>>(b->d_nodes, b->stats.nodes,
+      rebase_nodes_kernel<<<blocks_of(b->stats.nodes, 256), 256>>>(b->d_frames, b->stats.nodes,
                                                                     sc->d_nodes + m.node_off,
                                                                     static_cast<int32_t>(m.node_off),
                                                                     static_cast<int32_t>(m.tri_off));
@@ -270,7 +270,7 @@ int n2w_scene_info(const n2w_scene* scene, int* mesh_count, int64_t* nodes, int6
     if (nodes) *nodes = scene->nodes;
     if (triangles) *triangles = scene->tris;
     if (device_bytes) {
-      *device_bytes = scene->nodes * static_cast<int64_t>(sizeof(Node4)) +
+      *device_bytes = scene->nodes * static_cast<int64_t>(sizeof(FrameNode4)) +
                       scene->tris * static_cast<int64_t>(sizeof(TriRec)) + scene->slots * 4;
     }
   });

@@ -241,6 +241,7 @@ struct Collapser {
     }
     const int self = static_cast<int>(out.nodes.size());
     out.nodes.emplace_back();
+    out.ranges.push_back(TriRange{static_cast<int32_t>(out.tris.size()), 0});
     Node4 nd{};
     for (int k = 0; k < 4; ++k) {
       if (k < nk) {
@@ -264,6 +265,7 @@ struct Collapser {
       nd.child[k] = (c.left < 0) ? emit_leaf(c) : emit(kids[k], depth + 1);
     }
     out.nodes[self] = nd;
+    out.ranges[self].last = static_cast<int32_t>(out.tris.size());
     return self;
   }
 };

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
   bool busy = false, drained = false;
   dev::V3 p = dev::v3(0.0f, 0.0f, 0.0f);
   dev::ClosestHit hit;
-  hit.d2 = FLT_MAX;
+  hit.d2 = hit.lim = FLT_MAX;
   hit.id = INT32_MAX;
   hit.slot = -1;
   hit.cp = p;
@@ -88,6 +88,10 @@ __global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
   dev::LocalStack stack{stack_mem};
   uint32_t c_nodes = 0, c_tris = 0;
   bool overflow = false;
+  auto step = [&](bool& ov) {
+    if constexpr (kCount) return dev::trav_step_boxes(nodes, tris, p, hit, tv, stack, c_nodes, c_tris, ov);
+    else return dev::trav_step(nodes, tris, p, hit, tv, stack, c_nodes, c_tris, ov);
+  };
   for (;;) {
     while (!busy && !drained) {
       const unsigned claim = atomicAdd(&s_next, 1u);
@@ -109,7 +113,7 @@ __global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
         continue;
       }
       p = dev::v3(pt.x, pt.y, pt.z);
-      hit.d2 = FLT_MAX;
+      hit.d2 = hit.lim = FLT_MAX;
       hit.id = INT32_MAX;
       hit.slot = -1;
       hit.cp = dev::v3(0.0f, 0.0f, 0.0f);
@@ -139,7 +143,7 @@ __global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
         out_id[q] = hit.id == INT32_MAX ? -1 : hit.id;
         out_overflow[q] = kHandOff;
         busy = false;
-      } else if (!dev::trav_step(nodes, tris, p, hit, tv, stack, c_nodes, c_tris, ov)) {
+      } else if (!step(ov)) {
         out_d2[q] = hit.d2;
         out_cp[q] = n2w_vec3{hit.cp.x, hit.cp.y, hit.cp.z};
         out_id[q] = hit.id == INT32_MAX ? -1 : hit.id;
@@ -162,7 +166,7 @@ __global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
         out_id[q] = hit.id == INT32_MAX ? -1 : hit.id;
         out_overflow[q] = kHandOff;
         busy = false;
-      } else if (!dev::trav_step(nodes, tris, p, hit, tv, stack, c_nodes, c_tris, ov)) {
+      } else if (!step(ov)) {
         out_d2[q] = hit.d2;
         out_cp[q] = n2w_vec3{hit.cp.x, hit.cp.y, hit.cp.z};
         out_id[q] = hit.id == INT32_MAX ? -1 : hit.id;
@@ -225,18 +229,20 @@ __global__ void __launch_bounds__(32 * kFinishWarps) closest_point_finish_kernel
       if (lane < take) e = work[sp - take + lane];
       __syncwarp();
       sp -= take;
-      const float bound = __uint_as_float(static_cast<unsigned>(best_key >> 32));
+      const float bound = dev::prune_limit(__uint_as_float(static_cast<unsigned>(best_key >> 32)), p);
       int2 c0 = make_int2(kEmptyChild, 0), c1 = c0, c2 = c0, c3 = c0;
       int nc = 0;
       if (e.x != kEmptyChild && __int_as_float(e.y) <= bound) {
         if (e.x >= 0) {
           float4 lox, hix, loy, hiy, loz, hiz;
           int4 ch;
-          dev::load_node(nodes, e.x, lox, hix, loy, hiy, loz, hiz, ch);
-          float d[4] = {dev::box_d2(p, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x),
-                        dev::box_d2(p, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y),
-                        dev::box_d2(p, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z),
-                        dev::box_d2(p, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w)};
+          dev::V3 v;
+          dev::load_frame_node(nodes, e.x, lox, hix, loy, hiy, loz, hiz, ch, v);
+          const dev::V3 f = dev::to_frame(v, p);
+          float d[4] = {dev::box_d2_fast(f, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x),
+                        dev::box_d2_fast(f, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y),
+                        dev::box_d2_fast(f, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z),
+                        dev::box_d2_fast(f, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w)};
           const int r[4] = {ch.x, ch.y, ch.z, ch.w};
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -315,7 +321,7 @@ __global__ void __launch_bounds__(256) seed_grid_kernel(const float4* __restrict
                             __fadd_rn(loy, __fmul_rn(h, static_cast<float>(iy))),
                             __fadd_rn(loz, __fmul_rn(h, static_cast<float>(iz))));
   dev::ClosestHit hit;
-  hit.d2 = FLT_MAX;
+  hit.d2 = hit.lim = FLT_MAX;
   hit.id = INT32_MAX;
   hit.slot = 0;
   hit.cp = p;
@@ -358,7 +364,8 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
   // the kernel runs 256-thread blocks, each over its own range of the queries,
   // with the grid sized to the resident capacity of the GPU.
   (void)block_size;
-  const float4* nodes = reinterpret_cast<const float4*>(bvh.d_nodes);
+  const float4* nodes = d_nodes ? reinterpret_cast<const float4*>(bvh.d_nodes)
+                                : reinterpret_cast<const float4*>(bvh.d_frames);
   const float4* tris = reinterpret_cast<const float4*>(bvh.d_tris);
   const dev::SeedGrid sg = seed_grid_of(bvh);
   auto launch = [&](auto kern, const uint8_t* act, int* dn, int* dt) {
@@ -461,6 +468,7 @@ void check_query_args(const n2w_bvh* bvh, const void* pts, int n, const void* d2
 
 void release(n2w_bvh* b) {
   if (b->d_nodes) cudaFree(b->d_nodes);
+  if (b->d_frames) cudaFree(b->d_frames);
   if (b->d_tris) cudaFree(b->d_tris);
   if (b->d_seed) cudaFree(b->d_seed);
   delete b;
@@ -482,6 +490,7 @@ int n2w_bvh_create(const n2w_mesh* mesh, int leaf_size, const char* build_method
       N2W_CUDA(cudaMalloc(&b->d_tris, h.tris.size() * sizeof(TriRec)));
       N2W_CUDA(cudaMemcpy(b->d_nodes, h.nodes.data(), h.nodes.size() * sizeof(Node4), cudaMemcpyHostToDevice));
       N2W_CUDA(cudaMemcpy(b->d_tris, h.tris.data(), h.tris.size() * sizeof(TriRec), cudaMemcpyHostToDevice));
+      build_frames(*b, h);
       build_seed_grid(*b, *mesh, kSeedGridCells);
       N2W_CUDA(cudaDeviceSynchronize());
     } catch (...) {
@@ -490,6 +499,7 @@ int n2w_bvh_create(const n2w_mesh* mesh, int leaf_size, const char* build_method
     }
     const auto t1 = std::chrono::steady_clock::now();
     b->stats = host_stats(h, leaf_size, std::chrono::duration<double, std::milli>(t1 - t0).count());
+    b->stats.device_bytes += static_cast<int64_t>(h.nodes.size() * sizeof(FrameNode4));
     b->stats.device_bytes += static_cast<int64_t>(kSeedGridCells + 1) * (kSeedGridCells + 1) * (kSeedGridCells + 1) * 4;
     *out = b;
   });

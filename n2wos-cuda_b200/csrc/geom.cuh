@@ -213,8 +213,43 @@ __device__ __forceinline__ void load_node(const float4* __restrict__ nodes, int3
   ch = ldg_v8_first_int4(n + 6);
 }
 
+// load_node of a FrameNode4: the last load also brings the node's frame v.
+__device__ __forceinline__ void load_frame_node(const float4* __restrict__ frames, int32_t ref, float4& lox,
+                                                float4& hix, float4& loy, float4& hiy, float4& loz, float4& hiz,
+                                                int4& ch, V3& v) {
+  const float4* n = frames + static_cast<size_t>(ref) * 8;
+  float4 c, f;
+  ldg_v8f(n + 0, lox, hix);
+  ldg_v8f(n + 2, loy, hiy);
+  ldg_v8f(n + 4, loz, hiz);
+  ldg_v8f(n + 6, c, f);
+  ch = make_int4(__float_as_int(c.x), __float_as_int(c.y), __float_as_int(c.z), __float_as_int(c.w));
+  v = v3(f.x, f.y, f.z);
+}
+
+// p in the frame of a node (layout.h): p - v (v.p).
+__device__ __forceinline__ V3 to_frame(V3 v, V3 p) {
+  const float s = fmaf(v.z, p.z, fmaf(v.y, p.y, v.x * p.x));
+  return V3{fmaf(-s, v.x, p.x), fmaf(-s, v.y, p.y), fmaf(-s, v.z, p.z)};
+}
+
+// Largest computed box distance^2, in a node's frame, that a box holding a
+// triangle at computed distance^2 `best` can have.  With u = 2^-24 the frame's
+// coordinates of p are off by at most 7 u |p|, |v|^2 by 6 u and the distance
+// and its square by a few u more; the boxes carry the triangles' own rounding
+// (build_frames).  2^-20 |p|_1 = 16 u |p|_1 and a factor 1 + 2^-18 cover these
+// twice over, so no triangle that ties the best distance is pruned.  At most
+// FLT_MAX, which an empty slot's infinite distance exceeds.
+__device__ __forceinline__ float prune_limit(float best, V3 p) {
+  float s;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(s) : "f"(best));
+  s = fmaf(fabsf(p.x) + fabsf(p.y) + fabsf(p.z), 9.5367431640625e-07f, s);
+  return fminf(s * s * 1.000003814697265625f, FLT_MAX);
+}
+
 struct ClosestHit {
   float d2;
+  float lim;  // prune_limit of d2 (traversals over frame nodes)
   int id;    // original triangle id; INT32_MAX when nothing was found below the bound
   int slot;  // leaf-order index of that triangle (used to re-seed the next query)
   V3 cp;
@@ -246,6 +281,7 @@ __device__ __forceinline__ void test_slot_impl(const float4* __restrict__ tris, 
   const int id = __float_as_int(a.w);
   if (dd < hit.d2 || (dd == hit.d2 && id < hit.id)) {
     hit.d2 = dd;
+    hit.lim = prune_limit(dd, p);
     hit.id = id;
     hit.slot = slot;
     hit.cp = cp;
@@ -396,7 +432,7 @@ struct TravState {
 // lets lanes with short queries move on while others are still searching.
 // kFast selects the contracted-FP32 box and triangle routines (walker);
 // callers use the trav_step / trav_step_fast wrappers.
-template <bool kFast, class Stack>
+template <bool kFast, bool kFrame, class Stack>
 __device__ __forceinline__ bool trav_step_impl(const float4* __restrict__ nodes, const float4* __restrict__ tris,
                                           V3 p, ClosestHit& hit, TravState& t, Stack& stack,
                                           uint32_t& c_nodes, uint32_t& c_tris, bool& overflow) {
@@ -404,7 +440,7 @@ __device__ __forceinline__ bool trav_step_impl(const float4* __restrict__ nodes,
     bool found = false;
     while (t.sp > 0) {
       const int2 e = stack.pop(--t.sp);
-      if (__int_as_float(e.y) <= hit.d2) {
+      if (__int_as_float(e.y) <= (kFrame ? hit.lim : hit.d2)) {
         if (e.x >= 0) {
           t.ref = e.x;
         } else {
@@ -425,15 +461,18 @@ __device__ __forceinline__ bool trav_step_impl(const float4* __restrict__ nodes,
   }
   float4 lox, hix, loy, hiy, loz, hiz;
   int4 ch;
-  load_node(nodes, t.ref, lox, hix, loy, hiy, loz, hiz, ch);
-  ++c_nodes;
   float d0, d1, d2, d3;
-  if (kFast) {
-    d0 = box_d2_fast(p, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x);
-    d1 = box_d2_fast(p, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y);
-    d2 = box_d2_fast(p, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z);
-    d3 = box_d2_fast(p, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w);
+  ++c_nodes;
+  if (kFrame) {
+    V3 v;
+    load_frame_node(nodes, t.ref, lox, hix, loy, hiy, loz, hiz, ch, v);
+    const V3 q = to_frame(v, p);
+    d0 = box_d2_fast(q, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x);
+    d1 = box_d2_fast(q, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y);
+    d2 = box_d2_fast(q, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z);
+    d3 = box_d2_fast(q, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w);
   } else {
+    load_node(nodes, t.ref, lox, hix, loy, hiy, loz, hiz, ch);
     d0 = box_d2(p, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x);
     d1 = box_d2(p, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y);
     d2 = box_d2(p, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z);
@@ -445,7 +484,7 @@ __device__ __forceinline__ bool trav_step_impl(const float4* __restrict__ nodes,
   cswap(d0, r0, d2, r2);
   cswap(d1, r1, d3, r3);
   cswap(d1, r1, d2, r2);
-  const float best = hit.d2;
+  const float best = kFrame ? hit.lim : hit.d2;
   if (d3 <= best) {
     if (t.sp < kTraversalStack) stack.push(t.sp++, make_int2(r3, __float_as_int(d3)));
     else overflow = true;
@@ -470,15 +509,38 @@ __device__ __forceinline__ bool trav_step_impl(const float4* __restrict__ nodes,
   return true;
 }
 
-__device__ __forceinline__ bool trav_step(const float4* __restrict__ nodes, const float4* __restrict__ tris, V3 p,
+// trav_step: exact routines over frame nodes; trav_step_fast: the walker's;
+// trav_step_boxes: exact routines over the axis-aligned nodes (the counted
+// query, whose visit counts the CPU restatement reproduces).
+__device__ __forceinline__ bool trav_step(const float4* __restrict__ frames, const float4* __restrict__ tris, V3 p,
                                           ClosestHit& hit, TravState& t, LocalStack& stack, uint32_t& c_nodes,
                                           uint32_t& c_tris, bool& overflow) {
-  return trav_step_impl<false>(nodes, tris, p, hit, t, stack, c_nodes, c_tris, overflow);
+  return trav_step_impl<false, true>(frames, tris, p, hit, t, stack, c_nodes, c_tris, overflow);
 }
-__device__ __forceinline__ bool trav_step_fast(const float4* __restrict__ nodes, const float4* __restrict__ tris,
+__device__ __forceinline__ bool trav_step_fast(const float4* __restrict__ frames, const float4* __restrict__ tris,
                                                V3 p, ClosestHit& hit, TravState& t, LocalStack& stack,
                                                uint32_t& c_nodes, uint32_t& c_tris, bool& overflow) {
-  return trav_step_impl<true>(nodes, tris, p, hit, t, stack, c_nodes, c_tris, overflow);
+  return trav_step_impl<true, true>(frames, tris, p, hit, t, stack, c_nodes, c_tris, overflow);
+}
+__device__ __forceinline__ bool trav_step_boxes(const float4* __restrict__ nodes, const float4* __restrict__ tris,
+                                                V3 p, ClosestHit& hit, TravState& t, LocalStack& stack,
+                                                uint32_t& c_nodes, uint32_t& c_tris, bool& overflow) {
+  return trav_step_impl<false, false>(nodes, tris, p, hit, t, stack, c_nodes, c_tris, overflow);
+}
+
+// A whole query in one lane over the frame nodes: `hit` as for traverse.
+__device__ __forceinline__ void traverse_frames(const float4* __restrict__ frames, const float4* __restrict__ tris,
+                                                V3 p, ClosestHit& hit, TraversalStats& st, int32_t root) {
+  int2 stack_mem[kTraversalStack];
+  LocalStack stack{stack_mem};
+  TravState t{0, root, 0, 0};
+  uint32_t c_nodes = 0, c_tris = 0;
+  bool overflow = false;
+  while (trav_step(frames, tris, p, hit, t, stack, c_nodes, c_tris, overflow)) {
+  }
+  st.node_visits += static_cast<int>(c_nodes);
+  st.tri_tests += static_cast<int>(c_tris);
+  if (overflow) st.overflow = 1;
 }
 
 // +x ray / triangle test of the reference's slice mask

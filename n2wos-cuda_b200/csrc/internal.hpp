@@ -19,7 +19,8 @@ struct n2w_mesh {
 };
 
 struct n2w_bvh {
-  n2w::Node4* d_nodes = nullptr;
+  n2w::Node4* d_nodes = nullptr;         // axis-aligned boxes: ray parity, counted queries, the copied-out layout
+  n2w::FrameNode4* d_frames = nullptr;  // the same tree with boxes in per-node frames: closest-point traversals
   n2w::TriRec* d_tris = nullptr;
   int* d_seed = nullptr;  // seed grid: leaf slot of the nearest triangle per lattice node
   float seed_lo[3] = {0, 0, 0};
@@ -76,8 +77,12 @@ int guarded(F&& f) {
 }
 
 // ---- host BVH build (bvh_build.cpp) ----
+struct TriRange {
+  int32_t first, last;  // leaf-order triangles [first, last)
+};
 struct HostBvh {
   std::vector<Node4> nodes;
+  std::vector<TriRange> ranges;  // triangles below each node
   std::vector<TriRec> tris;
   int64_t binary_nodes = 0;
   int64_t leaves = 0;
@@ -91,6 +96,9 @@ n2w_bvh_stats host_stats(const HostBvh& h, int leaf_size, double ms);
 void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const uint8_t* d_active,
                           int n, float* d_d2, n2w_vec3* d_cp, int* d_id, int* d_overflow,
                           int* d_nodes, int* d_tris, int block_size, cudaStream_t stream);
+
+// Fills b.d_frames from the uploaded nodes and triangles.
+void build_frames(n2w_bvh& b, const HostBvh& h);
 
 void build_seed_grid(n2w_bvh& b, const n2w_mesh& mesh, int n);
 

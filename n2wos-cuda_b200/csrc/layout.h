@@ -41,6 +41,26 @@ struct alignas(128) Node4 {
 };
 static_assert(sizeof(Node4) == 128, "Node4 must be one 128-byte line");
 
+// The same 4-wide node with its child boxes in a frame of its own: the mirror
+// image q = p - v (v.p) with |v|^2 = 2 (v = 0: the axes themselves), chosen so
+// that the patch of surface below the node lies flat against an axis.  A
+// mirror is an isometry, so distances to the boxes are distances in space, and
+// three floats in the node's padding hold it.  Boxes around a flat patch in
+// such a frame are thin where axis-aligned ones are not, so far fewer children
+// lie within a query's best distance.
+struct alignas(128) FrameNode4 {
+  float lo_x[4];
+  float hi_x[4];
+  float lo_y[4];
+  float hi_y[4];
+  float lo_z[4];
+  float hi_z[4];
+  int32_t child[4];
+  float v[3];
+  int32_t pad;
+};
+static_assert(sizeof(FrameNode4) == sizeof(Node4), "both node arrays share their indices and loads");
+
 struct alignas(16) TriRec {
   float v0[3];
   int32_t id;

@@ -12,7 +12,7 @@
 #include "walker.cuh"
 
 struct n2w_scene {
-  n2w::Node4* d_nodes = nullptr;
+  n2w::FrameNode4* d_nodes = nullptr;
   n2w::TriRec* d_tris = nullptr;
   int* d_slots = nullptr;
   int64_t nodes = 0, tris = 0, slots = 0;

@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
   uint64_t wid = 0;
 
   dev::ClosestHit hit;
-  hit.d2 = FLT_MAX;
+  hit.d2 = hit.lim = FLT_MAX;
   hit.id = INT32_MAX;
   hit.slot = 0;
   hit.cp = x;
@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
       ++step;
       // Seed the next query with two real candidates (previous closest
       // triangle, seed-grid triangle at x); the exact answer is unchanged.
-      hit.d2 = FLT_MAX;
+      hit.d2 = hit.lim = FLT_MAX;
       hit.id = INT32_MAX;
       hit.cp = x;
       dev::test_slot_fast(a.tris, prev_slot, x, hit);
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(256) first_query_kernel(const float4* __restri
   const n2w_vec3 pt = points[i];
   const dev::V3 p = dev::v3(pt.x, pt.y, pt.z);
   dev::ClosestHit hit;
-  hit.d2 = FLT_MAX;
+  hit.d2 = hit.lim = FLT_MAX;
   hit.id = INT32_MAX;
   hit.slot = -1;
   hit.cp = p;
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(256) first_query_kernel(const float4* __restri
     dev::test_slot(tris, dev::seed_slot(grid, p), p, hit);
     ++st.tri_tests;
   }
-  dev::traverse<true>(nodes, tris, p, hit, st);
+  dev::traverse_frames(nodes, tris, p, hit, st, 0);
   cpd[i] = make_float4(hit.cp.x, hit.cp.y, hit.cp.z, hit.d2);
   ids[i] = make_int2(hit.id, hit.slot);
   if (counters) {
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(256) first_query_batch_kernel(const __grid_con
   const n2w_vec3 pt = I.points[i - I.point_base];
   const dev::V3 p = dev::v3(pt.x, pt.y, pt.z);
   dev::ClosestHit hit;
-  hit.d2 = FLT_MAX;
+  hit.d2 = hit.lim = FLT_MAX;
   hit.id = INT32_MAX;
   hit.slot = -1;
   hit.cp = p;
@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(256) first_query_batch_kernel(const __grid_con
     dev::test_slot(a.tris, dev::seed_slot(I.grid, p), p, hit);
     ++st.tri_tests;
   }
-  dev::traverse<true>(a.nodes, a.tris, p, hit, st, I.root);
+  dev::traverse_frames(a.nodes, a.tris, p, hit, st, I.root);
   cpd[i] = make_float4(hit.cp.x, hit.cp.y, hit.cp.z, hit.d2);
   ids[i] = make_int2(hit.id, hit.slot);
   if (a.counters) {
@@ -697,7 +697,7 @@ void validate_problem(const n2w_problem& p) {
 WalkArgs make_walk_args(const n2w_bvh& bvh, const n2w_problem& problem, const n2w_vec3* d_points,
                         int64_t point_count, const n2w_walk_options& o, uint32_t stream_tag) {
   WalkArgs a{};
-  a.nodes = reinterpret_cast<const float4*>(bvh.d_nodes);
+  a.nodes = reinterpret_cast<const float4*>(bvh.d_frames);
   a.tris = reinterpret_cast<const float4*>(bvh.d_tris);
   a.grid = seed_grid_of(bvh);
   for (int k = 0; k < 3; ++k) {
