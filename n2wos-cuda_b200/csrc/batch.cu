@@ -2,7 +2,7 @@
 // meshes, in ONE persistent walker launch.
 //
 //  * A scene merges the BVHs of several meshes into one device layout: node
-//    arrays, triangle arrays and seed-grid slots are concatenated and every
+//    arrays, triangle arrays and seed-grid cells are concatenated and every
 //    child reference / slot is rebased, so a walker only needs its instance's
 //    root node index to query its own mesh.
 //  * A batch is a fixed table of instances (mesh, problem, points, walks per
@@ -54,23 +54,29 @@ struct n2w_batch {
 namespace n2w {
 namespace {
 
+// A child reference in the merged scene's arrays.
+__device__ __forceinline__ int32_t rebase_ref(int32_t r, int32_t node_off, int32_t tri_off) {
+  if (r >= 0) return r + node_off;
+  return r == kEmptyChild ? r : leaf_ref(leaf_first(r) + tri_off, leaf_count(r));
+}
+
 __global__ void rebase_nodes_kernel(const FrameNode4* __restrict__ src, int64_t n, FrameNode4* __restrict__ dst,
                                     int32_t node_off, int32_t tri_off) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   FrameNode4 nd = src[i];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int32_t r = nd.child[c];
-    if (r >= 0) nd.child[c] = r + node_off;
-    else if (r != kEmptyChild) nd.child[c] = leaf_ref(leaf_first(r) + tri_off, leaf_count(r));
-  }
+  for (int c = 0; c < 4; ++c) nd.child[c] = rebase_ref(nd.child[c], node_off, tri_off);
   dst[i] = nd;
 }
 
-__global__ void rebase_slots_kernel(const int* __restrict__ src, int64_t n, int* __restrict__ dst, int32_t tri_off) {
+__global__ void rebase_cells_kernel(const int4* __restrict__ src, int64_t n, int4* __restrict__ dst, int32_t node_off,
+                                    int32_t tri_off) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = src[i] + tri_off;
+  if (i >= n) return;
+  const int4 c = src[i];
+  dst[i] = make_int4(c.x + tri_off, rebase_ref(c.y, node_off, tri_off), rebase_ref(c.z, node_off, tri_off),
+                     rebase_ref(c.w, node_off, tri_off));
 }
 
 // Zeroes the per-point accumulators of every instance (global point index i).
@@ -222,8 +228,8 @@ int n2w_scene_create(const n2w_bvh* const* bvhs, int count, n2w_scene** out) {
       sc->tris += b->stats.triangles;
       if (b->d_seed) {
         const int64_t s = static_cast<int64_t>(b->seed_n) + 1;
-        m.slot_off = sc->slots;
-        sc->slots += s * s * s;
+        m.cell_off = sc->cells;
+        sc->cells += s * s * s;
         for (int a = 0; a < 3; ++a) {
           m.seed_lo[a] = b->seed_lo[a];
           m.box_lo[a] = b->seed_lo[a];
@@ -237,7 +243,7 @@ int n2w_scene_create(const n2w_bvh* const* bvhs, int count, n2w_scene** out) {
                 "n2w_scene_create: merged scene exceeds 2^31 nodes or 2^28 triangles");
     N2W_CUDA(cudaMalloc(&sc->d_nodes, sizeof(FrameNode4) * sc->nodes));
     N2W_CUDA(cudaMalloc(&sc->d_tris, sizeof(TriRec) * sc->tris));
-    if (sc->slots) N2W_CUDA(cudaMalloc(&sc->d_slots, sizeof(int) * sc->slots));
+    if (sc->cells) N2W_CUDA(cudaMalloc(&sc->d_cells, sizeof(int4) * sc->cells));
     for (int k = 0; k < count; ++k) {
       const n2w_bvh* b = bvhs[k];
       const auto& m = sc->meshes[k];
@@ -248,9 +254,10 @@ int n2w_scene_create(const n2w_bvh* const* bvhs, int count, n2w_scene** out) {
       N2W_CUDA(cudaGetLastError());
       N2W_CUDA(cudaMemcpy(sc->d_tris + m.tri_off, b->d_tris, sizeof(TriRec) * b->stats.triangles,
                           cudaMemcpyDeviceToDevice));
-      if (m.slot_off >= 0) {
+      if (m.cell_off >= 0) {
         const int64_t s = static_cast<int64_t>(b->seed_n) + 1;
-        rebase_slots_kernel<<<blocks_of(s * s * s, 256), 256>>>(b->d_seed, s * s * s, sc->d_slots + m.slot_off,
+        rebase_cells_kernel<<<blocks_of(s * s * s, 256), 256>>>(b->d_seed, s * s * s, sc->d_cells + m.cell_off,
+                                                                static_cast<int32_t>(m.node_off),
                                                                 static_cast<int32_t>(m.tri_off));
         N2W_CUDA(cudaGetLastError());
       }
@@ -271,7 +278,7 @@ int n2w_scene_info(const n2w_scene* scene, int* mesh_count, int64_t* nodes, int6
     if (triangles) *triangles = scene->tris;
     if (device_bytes) {
       *device_bytes = scene->nodes * static_cast<int64_t>(sizeof(FrameNode4)) +
-                      scene->tris * static_cast<int64_t>(sizeof(TriRec)) + scene->slots * 4;
+                      scene->tris * static_cast<int64_t>(sizeof(TriRec)) + scene->cells * static_cast<int64_t>(sizeof(int4));
     }
   });
 }
@@ -280,7 +287,7 @@ void n2w_scene_destroy(n2w_scene* scene) {
   if (!scene) return;
   cudaFree(scene->d_nodes);
   cudaFree(scene->d_tris);
-  cudaFree(scene->d_slots);
+  cudaFree(scene->d_cells);
   delete scene;
 }
 

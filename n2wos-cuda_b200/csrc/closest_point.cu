@@ -17,7 +17,7 @@ namespace n2w {
 
 dev::SeedGrid seed_grid_of(const n2w_bvh& b) {
   dev::SeedGrid g;
-  g.slots = b.d_seed;
+  g.cells = b.d_seed;
   g.lo_x = b.seed_lo[0];
   g.lo_y = b.seed_lo[1];
   g.lo_z = b.seed_lo[2];
@@ -29,30 +29,27 @@ dev::SeedGrid seed_grid_of(const n2w_bvh& b) {
 namespace {
 
 // Persistent state machine, one lane per query.  Every iteration each busy
-// lane advances its query by ONE unit of traversal work (one 4-wide node
-// expansion or one triangle test, dev::trav_step), and a lane whose query is
-// complete writes it and takes the next query in the same iteration.  Each
+// lane advances its query by one step (dev::trav_triangle + dev::trav_node; the
+// counting variant by one unit of dev::trav_step_boxes), and a lane whose query
+// is complete writes it and takes the next query in the same iteration.  Each
 // block owns the contiguous range [b n / B, (b + 1) n / B) of the queries and
 // its lanes take them from a shared-memory counter as they finish, so a lane
 // that drew slow queries does not hold up queries that idle lanes of its
 // block could run (with a fixed grid-stride sequence, launches of ~1-2
-// queries per lane last as long as their unluckiest lane's pair).  Lanes therefore never wait for another lane's whole
-// traversal (one-query-per-thread loops leave ~3.6 of 32 lanes active on
-// incoherent queries); short work units keep the warp's two code paths
-// (node / triangle) busy.  The visit order, pruning and pushes are those of
-// dev::traverse, so results and node-visit / triangle-test counts are
-// identical to the one-query-per-thread traversal.
+// queries per lane last as long as their unluckiest lane's pair).  Lanes
+// therefore never wait for another lane's whole traversal (one-query-per-thread
+// loops leave ~3.6 of 32 lanes active on incoherent queries).
 constexpr int kQueryBlock = 256;
 // Traversal units (node expansions + triangle tests) a lane spends on one
 // query before handing it to the warp-cooperative finisher, when the launch
 // holds about one query per resident lane; the few queries far from the
 // surface in every direction (near the centre of a closed mesh) need
-// thousands, and one of them per lane would set the launch's length.  With
-// more queries per lane the lanes' totals even out and the budget grows in
-// proportion, so a full GPU hands off only the extreme queries (measured on
-// 262,144 / 4,194,304 uniform queries: budget 384 -> 1.4x / 1.0x the
-// single-phase rate; a fixed 192 -> 1.35x / 0.67x).
-constexpr uint32_t kQueryBudget = 384;
+// thousands against a mean of ~40, and one of them per lane would set the
+// launch's length.  With more queries per lane the lanes' totals even out and
+// the budget grows in proportion, so a full GPU hands off only the extreme
+// queries.  262,144 uniform queries: 399 / 392 / 423 / 451 / 481 us with a
+// budget of 96 / 128 / 192 / 256 / 384; 4,194,304: 4.78 ms with any of them.
+constexpr uint32_t kQueryBudget = 128;
 constexpr int kHandOff = 2;         // overflow-slot mark of a handed-off query
 constexpr int kFinishWarps = 4;     // warps per finisher block
 constexpr int kFinishStack = 2048;  // work-list entries per finisher warp (16 KiB)
@@ -62,6 +59,30 @@ constexpr int kFinishStack = 2048;  // work-list entries per finisher warp (16 K
 // 152.5 / 224.2 / 285.1 against 149.5 / 213.0 / 276.0 M queries/s at 131,072 /
 // 262,144 / 524,288 queries, equal at 1 M and 2 M, 391 against 405 at 4 M.
 constexpr int64_t kSmallLaunch = int64_t{1} << 21;
+
+// One lane's query in flight; step() returns false once it is complete.
+template <bool kCount>
+struct Search {
+  dev::FrameTrav t;
+  dev::FrameStack stack;
+  __device__ __forceinline__ void start(int4 cell) { t.start(cell, stack); }
+  __device__ __forceinline__ bool step(const float4* __restrict__ frames, const float4* __restrict__ tris, dev::V3 p,
+                                       dev::ClosestHit& hit, uint32_t& c_nodes, uint32_t& c_tris, bool& overflow) {
+    dev::trav_triangle<false>(tris, p, hit, t, stack, c_tris);
+    dev::trav_node(frames, p, hit, t, stack, c_nodes, overflow);
+    return !t.done();
+  }
+};
+template <>
+struct Search<true> {
+  dev::TravState t;
+  int2 stack[kTraversalStack];
+  __device__ __forceinline__ void start(int4) { t = dev::TravState{0, 0, 0, 0}; }  // every visit from the root counts
+  __device__ __forceinline__ bool step(const float4* __restrict__ nodes, const float4* __restrict__ tris, dev::V3 p,
+                                       dev::ClosestHit& hit, uint32_t& c_nodes, uint32_t& c_tris, bool& overflow) {
+    return dev::trav_step_boxes(nodes, tris, p, hit, t, stack, c_nodes, c_tris, overflow);
+  }
+};
 
 template <bool kMasked, bool kCount, int kMinBlocks>
 __global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
@@ -83,15 +104,9 @@ __global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
   hit.id = INT32_MAX;
   hit.slot = -1;
   hit.cp = p;
-  dev::TravState tv{0, kEmptyChild, 0, 0};
-  int2 stack_mem[kTraversalStack];
-  dev::LocalStack stack{stack_mem};
   uint32_t c_nodes = 0, c_tris = 0;
   bool overflow = false;
-  auto step = [&](bool& ov) {
-    if constexpr (kCount) return dev::trav_step_boxes(nodes, tris, p, hit, tv, stack, c_nodes, c_tris, ov);
-    else return dev::trav_step(nodes, tris, p, hit, tv, stack, c_nodes, c_tris, ov);
-  };
+  Search<kCount> search;
   for (;;) {
     while (!busy && !drained) {
       const unsigned claim = atomicAdd(&s_next, 1u);
@@ -119,22 +134,17 @@ __global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
       hit.cp = dev::v3(0.0f, 0.0f, 0.0f);
       c_nodes = c_tris = 0;
       overflow = false;
-      if (grid.slots) {
-        dev::test_slot(tris, dev::seed_slot(grid, p), p, hit);
+      int4 cell = make_int4(0, 0, kEmptyChild, kEmptyChild);  // the root
+      if (grid.cells) {
+        cell = dev::seed_cell(grid, p, 0);
+        dev::test_slot(tris, cell.x, p, hit);
         ++c_tris;
       }
-      tv.sp = 0;
-      tv.ref = 0;
-      tv.leaf_cur = tv.leaf_end = 0;
+      search.start(cell);
       busy = true;
     }
     if (!__any_sync(0xffffffffu, busy)) break;
-    // Two units per iteration, written out twice: the claim loop and the vote
-    // cost about as much as a unit (262,144 / 1,048,576 / 4,194,304 queries:
-    // 229.8 / 347.1 / 412.4 against 225.9 / 338.2 / 404.1 M queries/s with one;
-    // 229.8 / 345.8 / 410.9 as an unrolled loop).
     if (busy) {
-      bool ov = false;
       if (!kCount && budget && c_nodes + c_tris > budget) {
         // Over budget: hand the query to the warp-cooperative finisher with its
         // best so far (a bound on the answer) in its own output slots.
@@ -143,7 +153,7 @@ __global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
         out_id[q] = hit.id == INT32_MAX ? -1 : hit.id;
         out_overflow[q] = kHandOff;
         busy = false;
-      } else if (!step(ov)) {
+      } else if (!search.step(nodes, tris, p, hit, c_nodes, c_tris, overflow)) {
         out_d2[q] = hit.d2;
         out_cp[q] = n2w_vec3{hit.cp.x, hit.cp.y, hit.cp.z};
         out_id[q] = hit.id == INT32_MAX ? -1 : hit.id;
@@ -154,30 +164,6 @@ __global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
         }
         busy = false;
       }
-      if (ov) overflow = true;
-    }
-    if (busy) {
-      bool ov = false;
-      if (!kCount && budget && c_nodes + c_tris > budget) {
-        // Over budget: hand the query to the warp-cooperative finisher with its
-        // best so far (a bound on the answer) in its own output slots.
-        out_d2[q] = hit.d2;
-        out_cp[q] = n2w_vec3{hit.cp.x, hit.cp.y, hit.cp.z};
-        out_id[q] = hit.id == INT32_MAX ? -1 : hit.id;
-        out_overflow[q] = kHandOff;
-        busy = false;
-      } else if (!step(ov)) {
-        out_d2[q] = hit.d2;
-        out_cp[q] = n2w_vec3{hit.cp.x, hit.cp.y, hit.cp.z};
-        out_id[q] = hit.id == INT32_MAX ? -1 : hit.id;
-        out_overflow[q] = overflow ? 1 : 0;
-        if (kCount) {
-          out_nodes[q] = static_cast<int>(c_nodes);
-          out_tris[q] = static_cast<int>(c_tris);
-        }
-        busy = false;
-      }
-      if (ov) overflow = true;
     }
   }
 }
@@ -308,7 +294,7 @@ __global__ void __launch_bounds__(32 * kFinishWarps) closest_point_finish_kernel
 // Builds the seed grid: a cold exact query at every lattice node.
 __global__ void __launch_bounds__(256) seed_grid_kernel(const float4* __restrict__ nodes,
                                                         const float4* __restrict__ tris, float lox, float loy,
-                                                        float loz, float h, int n, int* __restrict__ slots,
+                                                        float loz, float h, int n, int4* __restrict__ cells,
                                                         int* __restrict__ overflow) {
   const int s = n + 1;
   const int64_t total = static_cast<int64_t>(s) * s * s;
@@ -327,7 +313,7 @@ __global__ void __launch_bounds__(256) seed_grid_kernel(const float4* __restrict
   hit.cp = p;
   dev::TraversalStats st{0, 0, 0};
   dev::traverse<false>(nodes, tris, p, hit, st);
-  slots[i] = hit.slot;
+  cells[i] = make_int4(hit.slot, 0, kEmptyChild, kEmptyChild);  // from the root until build_cell_entries
   if (st.overflow) atomicOr(overflow, 1);
 }
 
@@ -436,7 +422,7 @@ void build_seed_grid(n2w_bvh& b, const n2w_mesh& mesh, int n) {
   b.seed_h = h;
   b.seed_n = n;
   const int64_t total = static_cast<int64_t>(n + 1) * (n + 1) * (n + 1);
-  N2W_CUDA(cudaMalloc(&b.d_seed, total * sizeof(int)));
+  N2W_CUDA(cudaMalloc(&b.d_seed, total * sizeof(int4)));
   int* d_ov = nullptr;
   N2W_CUDA(cudaMalloc(&d_ov, sizeof(int)));
   N2W_CUDA(cudaMemset(d_ov, 0, sizeof(int)));
@@ -445,6 +431,7 @@ void build_seed_grid(n2w_bvh& b, const n2w_mesh& mesh, int n) {
       reinterpret_cast<const float4*>(b.d_nodes), reinterpret_cast<const float4*>(b.d_tris), b.seed_lo[0],
       b.seed_lo[1], b.seed_lo[2], h, n, b.d_seed, d_ov);
   N2W_CUDA(cudaGetLastError());
+  build_cell_entries(b);
   int ov = 0;
   N2W_CUDA(cudaMemcpy(&ov, d_ov, sizeof(int), cudaMemcpyDeviceToHost));
   cudaFree(d_ov);
@@ -500,7 +487,8 @@ int n2w_bvh_create(const n2w_mesh* mesh, int leaf_size, const char* build_method
     const auto t1 = std::chrono::steady_clock::now();
     b->stats = host_stats(h, leaf_size, std::chrono::duration<double, std::milli>(t1 - t0).count());
     b->stats.device_bytes += static_cast<int64_t>(h.nodes.size() * sizeof(FrameNode4));
-    b->stats.device_bytes += static_cast<int64_t>(kSeedGridCells + 1) * (kSeedGridCells + 1) * (kSeedGridCells + 1) * 4;
+    b->stats.device_bytes += static_cast<int64_t>(kSeedGridCells + 1) * (kSeedGridCells + 1) * (kSeedGridCells + 1) *
+                              static_cast<int64_t>(sizeof(int4));
     *out = b;
   });
 }
@@ -587,7 +575,7 @@ int n2w_bvh_seed_grid(const n2w_bvh* bvh, float* lo_out, float* h_out, int* n_ou
     if (n_out) *n_out = bvh->seed_n;
     if (slots_out) {
       const size_t s = static_cast<size_t>(bvh->seed_n) + 1;
-      N2W_CUDA(cudaMemcpy(slots_out, bvh->d_seed, s * s * s * sizeof(int), cudaMemcpyDeviceToHost));
+      copy_cell_slots(*bvh, static_cast<int64_t>(s * s * s), slots_out);
     }
   });
 }

@@ -22,7 +22,7 @@ struct n2w_bvh {
   n2w::Node4* d_nodes = nullptr;         // axis-aligned boxes: ray parity, counted queries, the copied-out layout
   n2w::FrameNode4* d_frames = nullptr;  // the same tree with boxes in per-node frames: closest-point traversals
   n2w::TriRec* d_tris = nullptr;
-  int* d_seed = nullptr;  // seed grid: leaf slot of the nearest triangle per lattice node
+  int4* d_seed = nullptr;  // seed grid: nearest triangle's leaf slot and start subtrees per lattice node (geom.cuh)
   float seed_lo[3] = {0, 0, 0};
   float seed_h = 0.0f;
   int seed_n = 0;
@@ -99,6 +99,11 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
 
 // Fills b.d_frames from the uploaded nodes and triangles.
 void build_frames(n2w_bvh& b, const HostBvh& h);
+
+// Fills the start subtrees of the seed grid's cells, whose slots are set.
+void build_cell_entries(n2w_bvh& b);
+// Host copy of the seed grid's n slots.
+void copy_cell_slots(const n2w_bvh& b, int64_t n, int* out);
 
 void build_seed_grid(n2w_bvh& b, const n2w_mesh& mesh, int n);
 

@@ -1,5 +1,5 @@
 // Merged multi-mesh device layout shared by batched launches and the serving
-// loop: concatenated 4-wide nodes, leaf-ordered triangles and seed-grid slots
+// loop: concatenated 4-wide nodes, leaf-ordered triangles and seed-grid cells
 // of several BVHs, with every index rebased, plus per-mesh metadata.
 #pragma once
 
@@ -14,11 +14,11 @@
 struct n2w_scene {
   n2w::FrameNode4* d_nodes = nullptr;
   n2w::TriRec* d_tris = nullptr;
-  int* d_slots = nullptr;
-  int64_t nodes = 0, tris = 0, slots = 0;
+  int4* d_cells = nullptr;
+  int64_t nodes = 0, tris = 0, cells = 0;
   struct MeshEntry {
     int32_t root = 0;
-    int64_t node_off = 0, tri_off = 0, slot_off = -1;
+    int64_t node_off = 0, tri_off = 0, cell_off = -1;
     float seed_lo[3] = {0, 0, 0};
     float seed_h = 0.0f;
     int seed_n = 0;
@@ -36,7 +36,7 @@ namespace n2w {
 inline void set_instance_geometry(BatchInst& I, const n2w_scene& sc, int mesh) {
   const auto& m = sc.meshes[mesh];
   I.root = m.root;
-  I.grid.slots = m.slot_off >= 0 ? sc.d_slots + m.slot_off : nullptr;
+  I.grid.cells = m.cell_off >= 0 ? sc.d_cells + m.cell_off : nullptr;
   I.grid.lo_x = m.seed_lo[0];
   I.grid.lo_y = m.seed_lo[1];
   I.grid.lo_z = m.seed_lo[2];

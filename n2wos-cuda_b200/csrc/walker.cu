@@ -202,9 +202,9 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
   hit.id = INT32_MAX;
   hit.slot = 0;
   hit.cp = x;
-  dev::TravState tv{0, kEmptyChild, 0, 0};
-  int2 stack_mem[kTraversalStack];
-  dev::LocalStack stack{stack_mem};
+  dev::FrameTrav tv;
+  tv.start(kEmptyChild);
+  dev::FrameStack stack;
 
   double acc_s = 0.0, acc_s2 = 0.0;
   uint32_t acc_n = 0, acc_forced = 0, acc_steps = 0;
@@ -354,17 +354,18 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
         if constexpr (kBatch) return a.insts[inst].grid;
         else return a.grid;
       }();
-      if (grid.slots) {
-        const int sg = dev::seed_slot(grid, x);
-        if (sg != prev_slot) {
-          dev::test_slot_fast(a.tris, sg, x, hit);
+      int root = 0;
+      if constexpr (kBatch) root = a.insts[inst].root;
+      if (grid.cells) {
+        const int4 cell = dev::seed_cell(grid, x, root);
+        if (cell.x != prev_slot) {
+          dev::test_slot_fast(a.tris, cell.x, x, hit);
           ++c_tris;
         }
+        tv.start(cell, stack);
+      } else {
+        tv.start(root);
       }
-      tv.sp = 0;
-      if constexpr (kBatch) tv.ref = a.insts[inst].root;
-      else tv.ref = 0;
-      tv.leaf_cur = tv.leaf_end = 0;
       querying = true;
     }
     // (3) flush finished (or abandoned) chunks' accumulators; always before the
@@ -442,31 +443,17 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
       const unsigned busy = __ballot_sync(0xffffffffu, querying);
       const unsigned waiting = __ballot_sync(0xffffffffu, !querying && alive);
       if (busy == 0 || __popc(waiting) >= a.regen) break;
-      // kUnits = 2 runs two units of traversal per vote, written out twice: the
-      // votes and the exit test cost about as much as a unit, and a lane that
-      // finishes on the first unit waits at most one unit longer (headline
-      // slice, same box: one unit 1,031, two 1,070, three 1,040 M
-      // walk-steps/s; the two units as an unrolled loop 1,054).  Compiled in,
-      // the second unit slows walks whose steps carry several source samples
-      // (16 per ball: 29.4 ns per walk with one unit, 31.4 with the second
-      // unit present even when it is skipped), so they run the kUnits = 1
-      // kernel.
       if (querying) {
         bool ov = false;
-        if (!dev::trav_step_fast(a.nodes, a.tris, x, hit, tv, stack, c_nodes, c_tris, ov)) querying = false;
+#pragma unroll
+        for (int u = 0; u < kUnits; ++u) {
+          dev::trav_triangle<true>(a.tris, x, hit, tv, stack, c_tris);
+          dev::trav_node(a.nodes, x, hit, tv, stack, c_nodes, ov);
+        }
+        querying = !tv.done();
         if (ov) {
           w_overflow = true;
           ++c_overflow;
-        }
-      }
-      if constexpr (kUnits == 2) {
-        if (querying) {
-          bool ov = false;
-          if (!dev::trav_step_fast(a.nodes, a.tris, x, hit, tv, stack, c_nodes, c_tris, ov)) querying = false;
-          if (ov) {
-            w_overflow = true;
-            ++c_overflow;
-          }
         }
       }
     }
@@ -511,11 +498,7 @@ __global__ void __launch_bounds__(256) first_query_kernel(const float4* __restri
   hit.slot = -1;
   hit.cp = p;
   dev::TraversalStats st{0, 0, 0};
-  if (grid.slots) {
-    dev::test_slot(tris, dev::seed_slot(grid, p), p, hit);
-    ++st.tri_tests;
-  }
-  dev::traverse_frames(nodes, tris, p, hit, st, 0);
+  dev::traverse_frames(nodes, tris, grid, p, hit, st, 0);
   cpd[i] = make_float4(hit.cp.x, hit.cp.y, hit.cp.z, hit.d2);
   ids[i] = make_int2(hit.id, hit.slot);
   if (counters) {
@@ -546,11 +529,7 @@ __global__ void __launch_bounds__(256) first_query_batch_kernel(const __grid_con
   hit.slot = -1;
   hit.cp = p;
   dev::TraversalStats st{0, 0, 0};
-  if (I.grid.slots) {
-    dev::test_slot(a.tris, dev::seed_slot(I.grid, p), p, hit);
-    ++st.tri_tests;
-  }
-  dev::traverse_frames(a.nodes, a.tris, p, hit, st, I.root);
+  dev::traverse_frames(a.nodes, a.tris, I.grid, p, hit, st, I.root);
   cpd[i] = make_float4(hit.cp.x, hit.cp.y, hit.cp.z, hit.d2);
   ids[i] = make_int2(hit.id, hit.slot);
   if (a.counters) {

@@ -35,7 +35,7 @@ struct alignas(16) BatchInst {
   int64_t point_count;
   int64_t chunk_base;           // first global chunk of this instance
   int64_t chunks_per_point;
-  dev::SeedGrid grid;           // slots already rebased into the merged scene
+  dev::SeedGrid grid;           // cells already rebased into the merged scene
   float box_lo[3], box_hi[3];   // domain box (walks never leave it)
   int32_t walks_per_point;
   int32_t root;                 // root node of this instance's mesh in the scene
