@@ -217,7 +217,7 @@ int n2w_scene_create(const n2w_bvh* const* bvhs, int count, n2w_scene** out) {
     sc->meshes.resize(count);
     for (int k = 0; k < count; ++k) {
       const n2w_bvh* b = bvhs[k];
-      N2W_REQUIRE(b && b->d_frames && b->d_tris, "n2w_scene_create: null BVH");
+      N2W_REQUIRE(b && b->d_frames && b->d_edges, "n2w_scene_create: null BVH");
       N2W_REQUIRE(b->device == sc->device, "n2w_scene_create: BVH on another device");
       auto& m = sc->meshes[k];
       m.node_off = sc->nodes;
@@ -242,7 +242,7 @@ int n2w_scene_create(const n2w_bvh* const* bvhs, int count, n2w_scene** out) {
     N2W_REQUIRE(sc->nodes < (int64_t{1} << 31) && sc->tris < (int64_t{1} << 28),
                 "n2w_scene_create: merged scene exceeds 2^31 nodes or 2^28 triangles");
     N2W_CUDA(cudaMalloc(&sc->d_nodes, sizeof(FrameNode4) * sc->nodes));
-    N2W_CUDA(cudaMalloc(&sc->d_tris, sizeof(TriRec) * sc->tris));
+    N2W_CUDA(cudaMalloc(&sc->d_tris, sizeof(TriEdges) * sc->tris));
     if (sc->cells) N2W_CUDA(cudaMalloc(&sc->d_cells, sizeof(int4) * sc->cells));
     for (int k = 0; k < count; ++k) {
       const n2w_bvh* b = bvhs[k];
@@ -252,7 +252,7 @@ int n2w_scene_create(const n2w_bvh* const* bvhs, int count, n2w_scene** out) {
                                                                     static_cast<int32_t>(m.node_off),
                                                                     static_cast<int32_t>(m.tri_off));
       N2W_CUDA(cudaGetLastError());
-      N2W_CUDA(cudaMemcpy(sc->d_tris + m.tri_off, b->d_tris, sizeof(TriRec) * b->stats.triangles,
+      N2W_CUDA(cudaMemcpy(sc->d_tris + m.tri_off, b->d_edges, sizeof(TriEdges) * b->stats.triangles,
                           cudaMemcpyDeviceToDevice));
       if (m.cell_off >= 0) {
         const int64_t s = static_cast<int64_t>(b->seed_n) + 1;
@@ -278,7 +278,7 @@ int n2w_scene_info(const n2w_scene* scene, int* mesh_count, int64_t* nodes, int6
     if (triangles) *triangles = scene->tris;
     if (device_bytes) {
       *device_bytes = scene->nodes * static_cast<int64_t>(sizeof(FrameNode4)) +
-                      scene->tris * static_cast<int64_t>(sizeof(TriRec)) + scene->cells * static_cast<int64_t>(sizeof(int4));
+                      scene->tris * static_cast<int64_t>(sizeof(TriEdges)) + scene->cells * static_cast<int64_t>(sizeof(int4));
     }
   });
 }

@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(256) seed_grid_kernel(const float4* __restrict
   hit.slot = 0;
   hit.cp = p;
   dev::TraversalStats st{0, 0, 0};
-  dev::traverse<false>(nodes, tris, p, hit, st);
+  dev::traverse(nodes, tris, p, hit, st);
   cells[i] = make_int4(hit.slot, 0, kEmptyChild, kEmptyChild);  // from the root until build_cell_entries
   if (st.overflow) atomicOr(overflow, 1);
 }
@@ -352,7 +352,7 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
   (void)block_size;
   const float4* nodes = d_nodes ? reinterpret_cast<const float4*>(bvh.d_nodes)
                                 : reinterpret_cast<const float4*>(bvh.d_frames);
-  const float4* tris = reinterpret_cast<const float4*>(bvh.d_tris);
+  const float4* tris = reinterpret_cast<const float4*>(bvh.d_edges);
   const dev::SeedGrid sg = seed_grid_of(bvh);
   auto launch = [&](auto kern, const uint8_t* act, int* dn, int* dt) {
     int occ = 0;
@@ -428,7 +428,7 @@ void build_seed_grid(n2w_bvh& b, const n2w_mesh& mesh, int n) {
   N2W_CUDA(cudaMemset(d_ov, 0, sizeof(int)));
   const int block = 256;
   seed_grid_kernel<<<static_cast<unsigned>((total + block - 1) / block), block>>>(
-      reinterpret_cast<const float4*>(b.d_nodes), reinterpret_cast<const float4*>(b.d_tris), b.seed_lo[0],
+      reinterpret_cast<const float4*>(b.d_nodes), reinterpret_cast<const float4*>(b.d_edges), b.seed_lo[0],
       b.seed_lo[1], b.seed_lo[2], h, n, b.d_seed, d_ov);
   N2W_CUDA(cudaGetLastError());
   build_cell_entries(b);
@@ -457,6 +457,7 @@ void release(n2w_bvh* b) {
   if (b->d_nodes) cudaFree(b->d_nodes);
   if (b->d_frames) cudaFree(b->d_frames);
   if (b->d_tris) cudaFree(b->d_tris);
+  if (b->d_edges) cudaFree(b->d_edges);
   if (b->d_seed) cudaFree(b->d_seed);
   delete b;
 }
@@ -477,6 +478,7 @@ int n2w_bvh_create(const n2w_mesh* mesh, int leaf_size, const char* build_method
       N2W_CUDA(cudaMalloc(&b->d_tris, h.tris.size() * sizeof(TriRec)));
       N2W_CUDA(cudaMemcpy(b->d_nodes, h.nodes.data(), h.nodes.size() * sizeof(Node4), cudaMemcpyHostToDevice));
       N2W_CUDA(cudaMemcpy(b->d_tris, h.tris.data(), h.tris.size() * sizeof(TriRec), cudaMemcpyHostToDevice));
+      build_edges(*b, static_cast<int64_t>(h.tris.size()));
       build_frames(*b, h);
       build_seed_grid(*b, *mesh, kSeedGridCells);
       N2W_CUDA(cudaDeviceSynchronize());
@@ -486,7 +488,7 @@ int n2w_bvh_create(const n2w_mesh* mesh, int leaf_size, const char* build_method
     }
     const auto t1 = std::chrono::steady_clock::now();
     b->stats = host_stats(h, leaf_size, std::chrono::duration<double, std::milli>(t1 - t0).count());
-    b->stats.device_bytes += static_cast<int64_t>(h.nodes.size() * sizeof(FrameNode4));
+    b->stats.device_bytes += static_cast<int64_t>(h.nodes.size() * sizeof(FrameNode4) + h.tris.size() * sizeof(TriEdges));
     b->stats.device_bytes += static_cast<int64_t>(kSeedGridCells + 1) * (kSeedGridCells + 1) * (kSeedGridCells + 1) *
                               static_cast<int64_t>(sizeof(int4));
     *out = b;

@@ -236,6 +236,23 @@ __global__ void __launch_bounds__(256) cell_entries_kernel(const float4* __restr
   cells[i] = make_int4(slot, e[0], e[1], e[2]);
 }
 
+__global__ void __launch_bounds__(256) edges_kernel(const TriRec* __restrict__ tris, int64_t n,
+                                                    TriEdges* __restrict__ out) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const TriRec t = tris[i];
+  TriEdges o;
+  o.id = t.id;
+  for (int k = 0; k < 3; ++k) {
+    o.a[k] = t.v0[k];
+    o.b[k] = t.v1[k];
+    o.c[k] = t.v2[k];
+    o.ab[k] = __fsub_rn(t.v1[k], t.v0[k]);
+    o.ac[k] = __fsub_rn(t.v2[k], t.v0[k]);
+  }
+  out[i] = o;
+}
+
 __global__ void __launch_bounds__(256) cell_slots_kernel(const int4* __restrict__ cells, int64_t n,
                                                          int* __restrict__ slots) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -247,7 +264,7 @@ __global__ void __launch_bounds__(256) cell_slots_kernel(const int4* __restrict_
 void build_cell_entries(n2w_bvh& b) {
   const int64_t s = b.seed_n + 1, total = s * s * s;
   cell_entries_kernel<<<static_cast<unsigned>((total + 255) / 256), 256>>>(
-      reinterpret_cast<const float4*>(b.d_frames), reinterpret_cast<const float4*>(b.d_tris), b.seed_lo[0],
+      reinterpret_cast<const float4*>(b.d_frames), reinterpret_cast<const float4*>(b.d_edges), b.seed_lo[0],
       b.seed_lo[1], b.seed_lo[2], b.seed_h, b.seed_n, b.d_seed);
   N2W_CUDA(cudaGetLastError());
 }
@@ -261,6 +278,12 @@ void copy_cell_slots(const n2w_bvh& b, int64_t n, int* out) {
   cudaFree(d);
   N2W_CUDA(l);
   N2W_CUDA(e);
+}
+
+void build_edges(n2w_bvh& b, int64_t triangles) {
+  N2W_CUDA(cudaMalloc(&b.d_edges, sizeof(TriEdges) * static_cast<size_t>(triangles)));
+  edges_kernel<<<static_cast<unsigned>((triangles + 255) / 256), 256>>>(b.d_tris, triangles, b.d_edges);
+  N2W_CUDA(cudaGetLastError());
 }
 
 void build_frames(n2w_bvh& b, const HostBvh& h) {

@@ -46,9 +46,8 @@ __device__ __forceinline__ float vdot(V3 a, V3 b) { return fa(fa(fm(a.x, b.x), f
 //   edge bc: b + (c-b)*((d4-d3)/((d4-d3)+(d5-d6)))
 //   face:    (a + ab*(vb*r)) + ac*(vc*r),  r = 1/((va+vb)+vc)
 //   vertex regions return the vertex itself.
-__device__ __forceinline__ V3 closest_point_triangle(V3 p, V3 a, V3 b, V3 c) {
-  const V3 ab = vsub(b, a);
-  const V3 ac = vsub(c, a);
+// The edges ab = b - a and ac = c - a come with the triangle (TriEdges).
+__device__ __forceinline__ V3 closest_point_triangle(V3 p, V3 a, V3 b, V3 c, V3 ab, V3 ac) {
   const V3 ap = vsub(p, a);
   const float d1 = vdot(ab, ap);
   const float d2 = vdot(ac, ap);
@@ -121,9 +120,7 @@ __device__ __forceinline__ V3 vmad_fast(V3 e, float s, V3 base) {
   return V3{fmaf(e.x, s, base.x), fmaf(e.y, s, base.y), fmaf(e.z, s, base.z)};
 }
 
-__device__ __forceinline__ V3 closest_point_triangle_fast(V3 p, V3 a, V3 b, V3 c) {
-  const V3 ab = vsub_fast(b, a);
-  const V3 ac = vsub_fast(c, a);
+__device__ __forceinline__ V3 closest_point_triangle_fast(V3 p, V3 a, V3 b, V3 c, V3 ab, V3 ac) {
   const V3 ap = vsub_fast(p, a);
   const float d1 = vdot_fast(ab, ap);
   const float d2 = vdot_fast(ac, ap);
@@ -261,24 +258,24 @@ struct ClosestHit {
 // triangle routine (walker); callers use the test_slot / test_slot_fast wrappers.
 template <bool kFast>
 __device__ __forceinline__ void test_slot_impl(const float4* __restrict__ tris, int slot, V3 p, ClosestHit& hit) {
-  // three 128-bit loads: a 256-bit + 128-bit split by record parity measured
-  // slower (the selects cost more than the saved load)
-  const float4* t = tris + static_cast<size_t>(slot) * 3;
-  const float4 a = __ldg(t + 0);
-  const float4 b = __ldg(t + 1);
-  const float4 c = __ldg(t + 2);
+  const float4* t = tris + static_cast<size_t>(slot) * 4;
+  float4 r0, r1, r2, r3;
+  ldg_v8f(t + 0, r0, r1);
+  ldg_v8f(t + 2, r2, r3);
+  const V3 a = v3(r0.x, r0.y, r0.z), ab = v3(r1.x, r1.y, r1.z), ac = v3(r1.w, r2.x, r2.y),
+           b = v3(r2.z, r2.w, r3.x), c = v3(r3.y, r3.z, r3.w);
   V3 cp;
   float dd;
   if (kFast) {
-    cp = closest_point_triangle_fast(p, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z));
+    cp = closest_point_triangle_fast(p, a, b, c, ab, ac);
     const V3 dv = vsub_fast(cp, p);
     dd = vdot_fast(dv, dv);
   } else {
-    cp = closest_point_triangle(p, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z));
+    cp = closest_point_triangle(p, a, b, c, ab, ac);
     const V3 dv = vsub(cp, p);
     dd = vdot(dv, dv);
   }
-  const int id = __float_as_int(a.w);
+  const int id = __float_as_int(r0.w);
   if (dd < hit.d2 || (dd == hit.d2 && id < hit.id)) {
     hit.d2 = dd;
     hit.lim = prune_limit(dd, p);
@@ -336,7 +333,6 @@ struct TraversalStats {
 // re-checked against the current best.  Candidates are any triangles whose box
 // distance is <= best_d2; `hit` must be initialised by the caller (cold query:
 // d2 = FLT_MAX, id = INT32_MAX; warm start: d2 = an upper bound).
-template <bool kCount>
 __device__ __forceinline__ void traverse(const float4* __restrict__ nodes,
                                          const float4* __restrict__ tris, V3 p, ClosestHit& hit,
                                          TraversalStats& st, int32_t root = 0) {
@@ -353,7 +349,6 @@ __device__ __forceinline__ void traverse(const float4* __restrict__ nodes,
       const float4 loz = __ldg(n + 4);
       const float4 hiz = __ldg(n + 5);
       const int4 ch = __ldg(reinterpret_cast<const int4*>(n + 6));
-      if (kCount) ++st.node_visits;
       float d0 = box_d2(p, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x);
       float d1 = box_d2(p, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y);
       float d2 = box_d2(p, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z);
@@ -381,23 +376,7 @@ __device__ __forceinline__ void traverse(const float4* __restrict__ nodes,
     } else if (ref != kEmptyChild) {
       const int first = leaf_first(ref);
       const int count = leaf_count(ref);
-      const float4* t = tris + static_cast<size_t>(first) * 3;
-      for (int i = 0; i < count; ++i) {
-        const float4 a = __ldg(t + 3 * i + 0);
-        const float4 b = __ldg(t + 3 * i + 1);
-        const float4 c = __ldg(t + 3 * i + 2);
-        if (kCount) ++st.tri_tests;
-        const V3 cp = closest_point_triangle(p, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z));
-        const V3 dv = vsub(cp, p);
-        const float dd = vdot(dv, dv);
-        const int id = __float_as_int(a.w);
-        if (dd < hit.d2 || (dd == hit.d2 && id < hit.id)) {
-          hit.d2 = dd;
-          hit.id = id;
-          hit.slot = first + i;
-          hit.cp = cp;
-        }
-      }
+      for (int i = 0; i < count; ++i) test_slot_impl<false>(tris, first + i, p, hit);
       ref = kEmptyChild;
     }
     if (ref == kEmptyChild) {

@@ -21,7 +21,8 @@ struct n2w_mesh {
 struct n2w_bvh {
   n2w::Node4* d_nodes = nullptr;         // axis-aligned boxes: ray parity, counted queries, the copied-out layout
   n2w::FrameNode4* d_frames = nullptr;  // the same tree with boxes in per-node frames: closest-point traversals
-  n2w::TriRec* d_tris = nullptr;
+  n2w::TriRec* d_tris = nullptr;        // leaf-ordered triangles: ray parity, the copied-out layout
+  n2w::TriEdges* d_edges = nullptr;     // the same triangles for the closest-point test
   int4* d_seed = nullptr;  // seed grid: nearest triangle's leaf slot and start subtrees per lattice node (geom.cuh)
   float seed_lo[3] = {0, 0, 0};
   float seed_h = 0.0f;
@@ -97,7 +98,8 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
                           int n, float* d_d2, n2w_vec3* d_cp, int* d_id, int* d_overflow,
                           int* d_nodes, int* d_tris, int block_size, cudaStream_t stream);
 
-// Fills b.d_frames from the uploaded nodes and triangles.
+// Fills b.d_edges and b.d_frames from the uploaded nodes and triangles.
+void build_edges(n2w_bvh& b, int64_t triangles);
 void build_frames(n2w_bvh& b, const HostBvh& h);
 
 // Fills the start subtrees of the seed grid's cells, whose slots are set.

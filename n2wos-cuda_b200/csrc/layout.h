@@ -71,6 +71,19 @@ struct alignas(16) TriRec {
 };
 static_assert(sizeof(TriRec) == 48, "TriRec must be 48 bytes");
 
+// A triangle as the closest-point test reads it: corner a with the original id,
+// the edges ab = b - a and ac = c - a (rounded once, as the test would round
+// them) and the corners b and c.  64 bytes, two aligned 256-bit loads.
+struct alignas(64) TriEdges {
+  float a[3];
+  int32_t id;
+  float ab[3];
+  float ac[3];
+  float b[3];
+  float c[3];
+};
+static_assert(sizeof(TriEdges) == 64, "TriEdges must be two 32-byte sectors");
+
 N2W_HD int32_t leaf_ref(int32_t first, int32_t count) { return ~((first << 3) | (count - 1)); }
 N2W_HD bool ref_is_leaf(int32_t r) { return r < 0 && r != kEmptyChild; }
 N2W_HD int32_t leaf_first(int32_t r) { return (~r) >> 3; }

@@ -13,7 +13,7 @@
 
 struct n2w_scene {
   n2w::FrameNode4* d_nodes = nullptr;
-  n2w::TriRec* d_tris = nullptr;
+  n2w::TriEdges* d_tris = nullptr;
   int4* d_cells = nullptr;
   int64_t nodes = 0, tris = 0, cells = 0;
   struct MeshEntry {

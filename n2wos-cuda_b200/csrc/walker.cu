@@ -677,7 +677,7 @@ WalkArgs make_walk_args(const n2w_bvh& bvh, const n2w_problem& problem, const n2
                         int64_t point_count, const n2w_walk_options& o, uint32_t stream_tag) {
   WalkArgs a{};
   a.nodes = reinterpret_cast<const float4*>(bvh.d_frames);
-  a.tris = reinterpret_cast<const float4*>(bvh.d_tris);
+  a.tris = reinterpret_cast<const float4*>(bvh.d_edges);
   a.grid = seed_grid_of(bvh);
   for (int k = 0; k < 3; ++k) {
     a.box_lo[k] = bvh.d_seed ? bvh.seed_lo[k] : -1.0e30f;

@@ -46,7 +46,7 @@ struct alignas(16) BatchInst {
 
 struct WalkArgs {
   const float4* nodes;  // FrameNode4 array
-  const float4* tris;
+  const float4* tris;   // TriEdges array
   dev::SeedGrid grid;
   float box_lo[3], box_hi[3];  // domain box: the mesh box grown by 20 % (walks never leave it)
   const n2w_vec3* points;
