@@ -116,13 +116,45 @@ __device__ __forceinline__ float ball_source(const n2w_problem& pb, uint32_t k0,
   return (R * R) * (1.0f / 6.0f) * f;
 }
 
+// Adds to point pid's FP64 totals (pid is the global point index; in batched
+// launches instance `inst` owns the accumulators).
+template <bool kBatch>
+__device__ __forceinline__ void add_point(int64_t pid, int inst, double s, double s2, uint32_t n, uint64_t steps,
+                                          uint32_t forced, const WalkArgs& a) {
+  double *sum = a.sum, *sum_sq = a.sum_sq;
+  uint32_t *count = a.count, *fc = a.forced;
+  uint64_t* st = a.steps;
+  if constexpr (kBatch) {
+    const BatchInst& I = a.insts[inst];
+    pid -= I.point_base;
+    sum = I.sum;
+    sum_sq = I.sum_sq;
+    count = I.count;
+    fc = I.forced;
+    st = I.steps;
+  }
+  atomicAdd(sum + pid, s);
+  atomicAdd(sum_sq + pid, s2);
+  atomicAdd(count + pid, n);
+  atomicAdd(reinterpret_cast<unsigned long long*>(st) + pid, static_cast<unsigned long long>(steps));
+  if (forced) atomicAdd(fc + pid, forced);
+}
+
 // Warp-collective flush of per-lane chunk accumulators into per-point FP64
-// totals: lanes are grouped by point id, each group is reduced by a shuffle
-// butterfly (non-members contribute zero) and its lowest lane issues the atomics.
+// totals.  Up to kDirectFlush lanes add their own (with single-walk chunks a
+// pass holds one or two, and a shuffle reduction costs about a hundred
+// instructions); more are grouped by point id, each group is reduced by a
+// shuffle butterfly (non-members contribute zero) and its lowest lane adds it.
+constexpr int kDirectFlush = 6;
+
 template <bool kBatch>
 __device__ __forceinline__ void warp_flush(bool want, int64_t pid, int inst, double s, double s2, uint32_t n,
                                            uint64_t steps, uint32_t forced, const WalkArgs& a) {
   unsigned pending = __ballot_sync(0xffffffffu, want);
+  if (__popc(pending) <= kDirectFlush) {
+    if (want) add_point<kBatch>(pid, inst, s, s2, n, steps, forced, a);
+    return;
+  }
   const int lane = threadIdx.x & 31;
   while (pending) {
     const int leader = __ffs(pending) - 1;
@@ -140,25 +172,7 @@ __device__ __forceinline__ void warp_flush(bool want, int64_t pid, int inst, dou
       vn += __shfl_xor_sync(0xffffffffu, vn, o);
       vf += __shfl_xor_sync(0xffffffffu, vf, o);
     }
-    if (kBatch) {
-      // pid is the global point index; the leader's instance owns the accumulators.
-      const int li = __shfl_sync(0xffffffffu, inst, leader);
-      if (lane == leader) {
-        const BatchInst& I = a.insts[li];
-        const int64_t q = lp - I.point_base;
-        atomicAdd(I.sum + q, vs);
-        atomicAdd(I.sum_sq + q, vs2);
-        atomicAdd(I.count + q, vn);
-        atomicAdd(reinterpret_cast<unsigned long long*>(I.steps) + q, vst);
-        atomicAdd(I.forced + q, vf);
-      }
-    } else if (lane == leader) {
-      atomicAdd(a.sum + lp, vs);
-      atomicAdd(a.sum_sq + lp, vs2);
-      atomicAdd(a.count + lp, vn);
-      atomicAdd(reinterpret_cast<unsigned long long*>(a.steps) + lp, vst);
-      atomicAdd(a.forced + lp, vf);
-    }
+    if (lane == leader) add_point<kBatch>(pid, inst, vs, vs2, vn, vst, vf, a);
     pending &= ~grp;
   }
 }
@@ -178,7 +192,7 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 //    warp returns to Phase A once `regen` lanes are waiting (or none is busy),
 //    so the walk updates run for many lanes at once and no lane waits for
 //    another lane's whole traversal.
-template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks, int kUnits = 1>
+template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks>
 __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(const __grid_constant__ WalkArgs a) {
   static_assert(!kBatch || (kOut == kOutStats && kWalk == N2W_WALK_PURE),
                 "batched launches run plain walks into per-point statistics");
@@ -234,139 +248,73 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
       exhausted = true;
       walk = walk_end;
     }
-    // (2) consume finished queries: score and finish, or move and seed the next
-    //     query.  A finished walk with more walks left in its chunk starts the
-    //     next one at once from the point's cached first query.
-    while (alive && !querying) {
+    // (2) finished queries: a walk that stops here is scored; with more walks left
+    //     in its chunk the lane starts the next one from the point's cached first
+    //     query.
+    float dist = 0.0f;
+    bool stop = false, forced = false;
+    auto at_end = [&]() {  // the current walk ends at its current query
+      dist = sqrtf(fmaxf(hit.d2, 0.0f));
+      forced = step - cont0 >= a.max_steps;  // steps since the walk (or its continuation) began
+      stop = dist <= a.eps || forced || !isfinite(dist) || hit.id == INT32_MAX;
+      return stop || (kWalk == N2W_WALK_PREFIX && step >= a.depth_m);
+    };
+    if (alive && !querying && at_end()) {
       ++c_queries;
-      const float d = sqrtf(fmaxf(hit.d2, 0.0f));
-      const int rel = step - cont0;  // steps since the walk (or its continuation) began
-      const bool forced = rel >= a.max_steps;
-      const bool stop = d <= a.eps || forced || !isfinite(d) || hit.id == INT32_MAX;
-      if (stop || (kWalk == N2W_WALK_PREFIX && step >= a.depth_m)) {
-        const float value = stop ? src + problem_u<float>(problem_of(), hit.cp.x, hit.cp.y, hit.cp.z) : src;
-        ++c_walks;
-        c_steps += static_cast<uint32_t>(step);
-        c_forced += forced ? 1u : 0u;
-        if (kOut == kOutStats) {
-          acc_s += static_cast<double>(value);
-          acc_s2 += static_cast<double>(value) * static_cast<double>(value);
-          ++acc_n;
-          acc_steps += static_cast<uint32_t>(step);
-          acc_forced += forced ? 1u : 0u;
+      const float value = stop ? src + problem_u<float>(problem_of(), hit.cp.x, hit.cp.y, hit.cp.z) : src;
+      ++c_walks;
+      c_steps += static_cast<uint32_t>(step);
+      c_forced += forced ? 1u : 0u;
+      if (kOut == kOutStats) {
+        acc_s += static_cast<double>(value);
+        acc_s2 += static_cast<double>(value) * static_cast<double>(value);
+        ++acc_n;
+        acc_steps += static_cast<uint32_t>(step);
+        acc_forced += forced ? 1u : 0u;
+      } else {
+        const uint64_t s = wid;
+        if (kOut == kOutSamples) {
+          a.s_value[s] = value;
         } else {
-          const uint64_t s = wid;
-          if (kOut == kOutSamples) {
-            a.s_value[s] = value;
+          // Prefix outputs (reference cubql_bvh.cu:1451-1606): X is X_m when the
+          // cache is needed, else the position where the walk stopped.
+          const bool needs = (kWalk == N2W_WALK_PREFIX) ? !stop : has_xm;
+          const dev::V3 xo = (kWalk == N2W_WALK_RESIDUAL && has_xm) ? xm : x;
+          a.p_inputs[3 * s + 0] = fminf(1.0f, fmaxf(0.0f, (xo.x - a.in_min[0]) / fmaxf(a.in_ext[0], 1.0e-6f)));
+          a.p_inputs[3 * s + 1] = fminf(1.0f, fmaxf(0.0f, (xo.y - a.in_min[1]) / fmaxf(a.in_ext[1], 1.0e-6f)));
+          a.p_inputs[3 * s + 2] = fminf(1.0f, fmaxf(0.0f, (xo.z - a.in_min[2]) / fmaxf(a.in_ext[2], 1.0e-6f)));
+          a.p_needs[s] = needs ? 1 : 0;
+          if (kWalk == N2W_WALK_PREFIX) {
+            a.p_boundary[s] = value;
           } else {
-            // Prefix outputs (reference cubql_bvh.cu:1451-1606): X is X_m when the
-            // cache is needed, else the position where the walk stopped.
-            const bool needs = (kWalk == N2W_WALK_PREFIX) ? !stop : has_xm;
-            const dev::V3 xo = (kWalk == N2W_WALK_RESIDUAL && has_xm) ? xm : x;
-            a.p_inputs[3 * s + 0] = fminf(1.0f, fmaxf(0.0f, (xo.x - a.in_min[0]) / fmaxf(a.in_ext[0], 1.0e-6f)));
-            a.p_inputs[3 * s + 1] = fminf(1.0f, fmaxf(0.0f, (xo.y - a.in_min[1]) / fmaxf(a.in_ext[1], 1.0e-6f)));
-            a.p_inputs[3 * s + 2] = fminf(1.0f, fmaxf(0.0f, (xo.z - a.in_min[2]) / fmaxf(a.in_ext[2], 1.0e-6f)));
-            a.p_needs[s] = needs ? 1 : 0;
-            if (kWalk == N2W_WALK_PREFIX) {
-              a.p_boundary[s] = value;
-            } else {
-              a.p_boundary[s] = needs ? am : value;
-              a.p_cont[s] = needs ? (value - am) : value;
-            }
+            a.p_boundary[s] = needs ? am : value;
+            a.p_cont[s] = needs ? (value - am) : value;
           }
-          a.s_steps[s] = step;
-          a.s_forced[s] = forced ? 1 : 0;
-          a.s_overflow[s] = w_overflow ? 1 : 0;
         }
-        ++walk;
-        if (walk < walk_end) {
-          // next walk of the same chunk: same point, cached first query
-          const n2w_vec3 p0 = start_point();
-          x = dev::v3(p0.x, p0.y, p0.z);
-          src = 0.0f;
-          step = 0;
-          cont0 = 0;
-          has_xm = false;
-          w_overflow = false;
-          ++wid;
-          const float4 c = __ldg(a.first_cpd + pid);
-          const int2 ii = __ldg(a.first_ids + pid);
-          hit.cp = dev::v3(c.x, c.y, c.z);
-          hit.d2 = c.w;
-          hit.id = ii.x;
-          hit.slot = ii.y;
-        } else {
-          alive = false;
-        }
-        continue;
+        a.s_steps[s] = step;
+        a.s_forced[s] = forced ? 1 : 0;
+        a.s_overflow[s] = w_overflow ? 1 : 0;
       }
-      if (kWalk == N2W_WALK_RESIDUAL && step == a.depth_m && !has_xm) {
-        // X_m reached: remember it and the prefix source; the continuation gets a
-        // fresh max_steps budget like the reference's nc_wos_from_point(X_m).
-        xm = x;
-        am = src;
-        has_xm = true;
-        cont0 = step;
-      }
-      const float R = a.step_scale * d;
-      uint32_t k0 = a.k0, k1 = a.k1;
-      if constexpr (kBatch) {
-        k0 = a.insts[inst].k0;
-        k1 = a.insts[inst].k1;
-      }
-      const U4 r = philox4x32_10(U4{static_cast<uint32_t>(wid), static_cast<uint32_t>(wid >> 32),
-                                    static_cast<uint32_t>(step), 0u},
-                                 k0, k1);
-      const dev::V3 dir = unit_sphere(r.x, r.y);
-      if constexpr (kBatch) {
-        const BatchInst& I = a.insts[inst];
-        if (I.has_source) src += ball_source(*I.problem, k0, k1, I.source_center, I.source_samples, x, R, wid, step, r.z);
+      ++walk;
+      if (walk < walk_end) {
+        // next walk of the same chunk: same point, cached first query
+        const n2w_vec3 p0 = start_point();
+        x = dev::v3(p0.x, p0.y, p0.z);
+        src = 0.0f;
+        step = 0;
+        cont0 = 0;
+        has_xm = false;
+        w_overflow = false;
+        ++wid;
+        const float4 c = __ldg(a.first_cpd + pid);
+        const int2 ii = __ldg(a.first_ids + pid);
+        hit.cp = dev::v3(c.x, c.y, c.z);
+        hit.d2 = c.w;
+        hit.id = ii.x;
+        hit.slot = ii.y;
       } else {
-        if (a.has_source) src += ball_source(a.problem, k0, k1, a.source_center, a.source_samples, x, R, wid, step, r.z);
+        alive = false;
       }
-      const int prev_slot = hit.slot;
-      const dev::V3 xn = dev::v3(x.x + R * dir.x, x.y + R * dir.y, x.z + R * dir.z);
-      const float* blo = a.box_lo;
-      const float* bhi = a.box_hi;
-      if constexpr (kBatch) {
-        blo = a.insts[inst].box_lo;
-        bhi = a.insts[inst].box_hi;
-      }
-      if (!(xn.x >= blo[0] && xn.x <= bhi[0] && xn.y >= blo[1] && xn.y <= bhi[1] && xn.z >= blo[2] &&
-            xn.z <= bhi[2])) {
-        // A walk from an interior point stays inside the mesh; leaving the
-        // domain box means the start point was outside (a misclassified sample).
-        // Stop it as forced, scored at the current closest point, instead of
-        // letting it wander the unbounded exterior.
-        step = cont0 + a.max_steps;
-        continue;
-      }
-      x = xn;
-      ++step;
-      // Seed the next query with two real candidates (previous closest
-      // triangle, seed-grid triangle at x); the exact answer is unchanged.
-      hit.d2 = hit.lim = FLT_MAX;
-      hit.id = INT32_MAX;
-      hit.cp = x;
-      dev::test_slot_fast(a.tris, prev_slot, x, hit);
-      ++c_tris;
-      const dev::SeedGrid& grid = [&]() -> const dev::SeedGrid& {
-        if constexpr (kBatch) return a.insts[inst].grid;
-        else return a.grid;
-      }();
-      int root = 0;
-      if constexpr (kBatch) root = a.insts[inst].root;
-      if (grid.cells) {
-        const int4 cell = dev::seed_cell(grid, x, root);
-        if (cell.x != prev_slot) {
-          dev::test_slot_fast(a.tris, cell.x, x, hit);
-          ++c_tris;
-        }
-        tv.start(cell, stack);
-      } else {
-        tv.start(root);
-      }
-      querying = true;
     }
     // (3) flush finished (or abandoned) chunks' accumulators; always before the
     //     exit test below, so nothing accumulated is ever dropped.
@@ -438,6 +386,78 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
     }
     if (!__any_sync(0xffffffffu, alive)) break;
 
+    // (5) move: every lane whose walk goes on, those that have just started one
+    //     included, takes its step in this one pass (a finished lane that looped
+    //     for its next walk's step ran the whole pass again, nearly alone).  A walk
+    //     that ends at its first query waits for the next Phase A.
+    if (alive && !querying && !at_end()) {
+      ++c_queries;
+      if (kWalk == N2W_WALK_RESIDUAL && step == a.depth_m && !has_xm) {
+        // X_m reached: remember it and the prefix source; the continuation gets a
+        // fresh max_steps budget like the reference's nc_wos_from_point(X_m).
+        xm = x;
+        am = src;
+        has_xm = true;
+        cont0 = step;
+      }
+      const float R = a.step_scale * dist;
+      uint32_t k0 = a.k0, k1 = a.k1;
+      if constexpr (kBatch) {
+        k0 = a.insts[inst].k0;
+        k1 = a.insts[inst].k1;
+      }
+      const U4 r = philox4x32_10(U4{static_cast<uint32_t>(wid), static_cast<uint32_t>(wid >> 32),
+                                    static_cast<uint32_t>(step), 0u},
+                                 k0, k1);
+      const dev::V3 dir = unit_sphere(r.x, r.y);
+      if constexpr (kBatch) {
+        const BatchInst& I = a.insts[inst];
+        if (I.has_source) src += ball_source(*I.problem, k0, k1, I.source_center, I.source_samples, x, R, wid, step, r.z);
+      } else {
+        if (a.has_source) src += ball_source(a.problem, k0, k1, a.source_center, a.source_samples, x, R, wid, step, r.z);
+      }
+      const int prev_slot = hit.slot;
+      const dev::V3 xn = dev::v3(x.x + R * dir.x, x.y + R * dir.y, x.z + R * dir.z);
+      const float* blo = a.box_lo;
+      const float* bhi = a.box_hi;
+      if constexpr (kBatch) {
+        blo = a.insts[inst].box_lo;
+        bhi = a.insts[inst].box_hi;
+      }
+      if (!(xn.x >= blo[0] && xn.x <= bhi[0] && xn.y >= blo[1] && xn.y <= bhi[1] && xn.z >= blo[2] &&
+            xn.z <= bhi[2])) {
+        // A walk from an interior point stays inside the mesh; leaving the
+        // domain box means the start point was outside (a misclassified sample).
+        // Stop it as forced, scored at the current closest point, instead of
+        // letting it wander the unbounded exterior.
+        step = cont0 + a.max_steps;
+      } else {
+        x = xn;
+        ++step;
+        // Seed the next query with two real candidates (previous closest
+        // triangle, seed-grid triangle at x); the exact answer is unchanged.
+        hit.d2 = hit.lim = FLT_MAX;
+        hit.id = INT32_MAX;
+        hit.cp = x;
+        const dev::SeedGrid& grid = [&]() -> const dev::SeedGrid& {
+          if constexpr (kBatch) return a.insts[inst].grid;
+          else return a.grid;
+        }();
+        int root = 0;
+        if constexpr (kBatch) root = a.insts[inst].root;
+        int4 cell = make_int4(prev_slot, root, kEmptyChild, kEmptyChild);
+        if (grid.cells) cell = dev::seed_cell(grid, x, root);
+        dev::test_slot_fast(a.tris, prev_slot, x, hit);
+        ++c_tris;
+        if (cell.x != prev_slot) {
+          dev::test_slot_fast(a.tris, cell.x, x, hit);
+          ++c_tris;
+        }
+        tv.start(cell, stack);
+        querying = true;
+      }
+    }
+
     // ================= Phase B =================
     for (;;) {
       const unsigned busy = __ballot_sync(0xffffffffu, querying);
@@ -445,11 +465,8 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
       if (busy == 0 || __popc(waiting) >= a.regen) break;
       if (querying) {
         bool ov = false;
-#pragma unroll
-        for (int u = 0; u < kUnits; ++u) {
-          dev::trav_triangle<true>(a.tris, x, hit, tv, stack, c_tris);
-          dev::trav_node(a.nodes, x, hit, tv, stack, c_nodes, ov);
-        }
+        dev::trav_triangle<true>(a.tris, x, hit, tv, stack, c_tris);
+        dev::trav_node(a.nodes, x, hit, tv, stack, c_nodes, ov);
         querying = !tv.done();
         if (ov) {
           w_overflow = true;
@@ -601,9 +618,9 @@ __global__ void combine_kernel(const float* __restrict__ cache, const float* __r
 // ---- host side -----------------------------------------------------------
 namespace {
 
-template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks, int kUnits = 1>
+template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks>
 void launch_walker(const WalkArgs& a, int block, int blocks_per_sm, cudaStream_t stream) {
-  auto kern = walker_kernel<kOut, kWalk, kBatch, kMinBlocks, kUnits>;
+  auto kern = walker_kernel<kOut, kWalk, kBatch, kMinBlocks>;
   int occ = 0;
   N2W_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, block, 0));
   if (occ < 1) occ = 1;
@@ -687,7 +704,8 @@ WalkArgs make_walk_args(const n2w_bvh& bvh, const n2w_problem& problem, const n2
   a.walks_per_point = o.walks_per_point;
   a.chunk = o.chunk > 0 ? std::min(o.chunk, o.walks_per_point) : std::min(kDefaultChunk, o.walks_per_point);
   a.chunks_per_point = (o.walks_per_point + a.chunk - 1) / a.chunk;
-  a.regen = o.regen_threshold > 0 ? o.regen_threshold : kDefaultRegen;
+  const bool many_samples = problem_has_source(problem) && problem.source_samples >= kManySamples;
+  a.regen = o.regen_threshold > 0 ? o.regen_threshold : (many_samples ? kManySamplesRegen : kDefaultRegen);
   a.total_chunks = point_count * a.chunks_per_point;
   a.max_steps = o.max_steps;
   a.depth_m = o.depth_m;
@@ -734,11 +752,7 @@ void run_walker(WalkArgs& a, int64_t point_count, int out_kind, int walk_mode, c
     N2W_CUDA(cudaGetLastError());
   }
   const int block = o.block_size > 0 ? o.block_size : kDefaultWalkerThreads;
-  if (out_kind == kOutStats) {
-    // two traversal units per vote unless the steps carry several source samples
-    if (a.has_source && a.source_samples > 1) launch_walker<kOutStats, N2W_WALK_PURE>(a, block, o.blocks_per_sm, stream);
-    else launch_walker<kOutStats, N2W_WALK_PURE, false, kWalkerMinBlocks, 2>(a, block, o.blocks_per_sm, stream);
-  }
+  if (out_kind == kOutStats) launch_walker<kOutStats, N2W_WALK_PURE>(a, block, o.blocks_per_sm, stream);
   else if (out_kind == kOutSamples) launch_walker<kOutSamples, N2W_WALK_PURE>(a, block, o.blocks_per_sm, stream);
   else if (walk_mode == N2W_WALK_PREFIX) launch_walker<kOutPrefix, N2W_WALK_PREFIX>(a, block, o.blocks_per_sm, stream);
   else launch_walker<kOutPrefix, N2W_WALK_RESIDUAL>(a, block, o.blocks_per_sm, stream);

@@ -26,7 +26,15 @@ constexpr int kDefaultWalkerThreads = 128;
 // 364.6 / 365.0 ms for 40,000 x 1,024, where the tail no longer shows: the queue
 // pops and per-point flushes of single walks cost nothing that can be measured.
 constexpr int kDefaultChunk = 1;
-constexpr int kDefaultRegen = 12;
+// Waiting lanes that make a warp leave the traversal for the walk update: more
+// lanes share the update, fewer traverse meanwhile.  8 / 12 / 14 / 16 / 20:
+// 47.8 / 46.3 / 46.2 / 46.2 / 47.2 ms (Poisson slice, 5.1 M walks), 39.2 / 37.9 /
+// 37.5 / 37.4 / 37.4 ms (batched instances).  With several source samples per
+// ball the update is the longer part: 16 samples, 8 / 12 / 16 / 20 / 24 / 28:
+// 21.6 / 18.3 / 16.9 / 16.3 / 16.3 / 17.1 ms.
+constexpr int kDefaultRegen = 16;
+constexpr int kManySamples = 4;
+constexpr int kManySamplesRegen = 20;
 
 // One instance of a batched launch: its geometry inside the merged scene, its
 // problem, its points and accumulators, and its slice of the global chunk queue.
