@@ -12,6 +12,7 @@
 
 #include "geom.cuh"
 #include "internal.hpp"
+#include "warp_search.cuh"
 
 namespace n2w {
 
@@ -51,8 +52,12 @@ constexpr int kQueryBlock = 256;
 // budget of 96 / 128 / 192 / 256 / 384; 4,194,304: 4.78 ms with any of them.
 constexpr uint32_t kQueryBudget = 128;
 constexpr int kHandOff = 2;         // overflow-slot mark of a handed-off query
-constexpr int kFinishWarps = 4;     // warps per finisher block
-constexpr int kFinishStack = 2048;  // work-list entries per finisher warp (16 KiB)
+// Launches of at most this many queries give each query a warp: with a lane per
+// query a launch lasts as long as its slowest serial search, whatever its size.
+// Lane / warp per query, uniform points, 81,920 triangles: 71 / 11 us (40
+// queries), 126 / 12 (1,000), 144 / 26 (4,000), 151 / 74 (16,000), 153 / 141
+// (32,000), 374 / 1,076 (262,144).
+constexpr int kWarpQueries = 32768;
 // Resident blocks per SM the traversal is compiled for (kMinBlocks).  Launches
 // of up to a few queries per lane run faster with 4 (up to 64 registers, no
 // spills) and larger ones with 5 (more warps to hide load latency): measured
@@ -168,126 +173,75 @@ __global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
   }
 }
 
-// Warp-cooperative finisher for the queries that ran over the per-lane
-// budget (marked kHandOff in their overflow slot): one warp per group of 32
-// consecutive queries takes its marked queries one at a time and traverses
-// the BVH from the root with the lane's best so far as the bound.  A
-// shared-memory work list of (node or leaf, box distance) entries feeds the 32
-// lanes: each iteration every lane takes one entry, expands a node (children
-// whose box is within the warp's best are pushed) or tests a leaf's
-// triangles, and the warp's best (d2, id) -- a 64-bit key, lowest d2 then
-// lowest id -- is the minimum over lanes.  Pruning is conservative, so the
-// answer is the exact one a single-lane traversal gives.  Blocks whose groups
-// hold no marked query exit at once, so the block scheduler balances the work.
-__device__ __forceinline__ unsigned long long hit_key(float d2, int id) {
-  return (static_cast<unsigned long long>(__float_as_uint(d2)) << 32) | static_cast<unsigned>(id);
-}
-
-__global__ void __launch_bounds__(32 * kFinishWarps) closest_point_finish_kernel(
-    const float4* __restrict__ nodes, const float4* __restrict__ tris, const n2w_vec3* __restrict__ points, int n,
-    float* __restrict__ out_d2, n2w_vec3* __restrict__ out_cp, int* __restrict__ out_id,
-    int* __restrict__ out_overflow) {
+// Finisher for the queries that ran over the per-lane budget (marked kHandOff in
+// their overflow slot): one warp per group of 32 consecutive queries takes its
+// marked queries one at a time and searches again (warp_search.cuh) with the
+// lane's best so far as the bound.  Blocks whose groups hold no marked query
+// exit at once, so the block scheduler balances the work.
+__global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) closest_point_finish_kernel(
+    const float4* __restrict__ nodes, const float4* __restrict__ tris, const dev::SeedGrid grid,
+    const n2w_vec3* __restrict__ points, int n, float* __restrict__ out_d2, n2w_vec3* __restrict__ out_cp,
+    int* __restrict__ out_id, int* __restrict__ out_overflow) {
   extern __shared__ int2 s_work[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  int2* work = s_work + warp * kFinishStack;
-  const int64_t q0 = (static_cast<int64_t>(blockIdx.x) * kFinishWarps + warp) * 32;
+  int2* work = s_work + warp * dev::kWarpList;
+  const int64_t q0 = (static_cast<int64_t>(blockIdx.x) * dev::kWarpsPerBlock + warp) * 32;
   if (q0 >= n) return;
   const int64_t mine = q0 + lane;
   unsigned pending = __ballot_sync(0xffffffffu, mine < n && out_overflow[mine] == kHandOff);
   while (pending) {
     const int q = static_cast<int>(q0) + __ffs(pending) - 1;
     pending &= pending - 1;
-    const n2w_vec3 pt = points[q];
+    const n2w_vec3 pt = points[q], c0 = out_cp[q];
     const dev::V3 p = dev::v3(pt.x, pt.y, pt.z);
     const int id0 = out_id[q];
-    const unsigned long long start_key = hit_key(out_d2[q], id0 < 0 ? INT32_MAX : id0);
-    unsigned long long best_key = start_key;  // warp-uniform
-    unsigned long long my_key = start_key;
-    dev::V3 my_cp = p;
-    bool dropped = false;  // warp-uniform: the work list was full
-    if (lane == 0) work[0] = make_int2(0, __float_as_int(0.0f));
-    int sp = 1;  // warp-uniform
-    __syncwarp();
-    while (sp > 0) {
-      const int take = min(sp, 32);
-      int2 e = make_int2(kEmptyChild, 0);
-      if (lane < take) e = work[sp - take + lane];
-      __syncwarp();
-      sp -= take;
-      const float bound = dev::prune_limit(__uint_as_float(static_cast<unsigned>(best_key >> 32)), p);
-      int2 c0 = make_int2(kEmptyChild, 0), c1 = c0, c2 = c0, c3 = c0;
-      int nc = 0;
-      if (e.x != kEmptyChild && __int_as_float(e.y) <= bound) {
-        if (e.x >= 0) {
-          float4 lox, hix, loy, hiy, loz, hiz;
-          int4 ch;
-          dev::V3 v;
-          dev::load_frame_node(nodes, e.x, lox, hix, loy, hiy, loz, hiz, ch, v);
-          const dev::V3 f = dev::to_frame(v, p);
-          float d[4] = {dev::box_d2_fast(f, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x),
-                        dev::box_d2_fast(f, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y),
-                        dev::box_d2_fast(f, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z),
-                        dev::box_d2_fast(f, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w)};
-          const int r[4] = {ch.x, ch.y, ch.z, ch.w};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if (r[k] != kEmptyChild && d[k] <= bound) {
-              const int2 ce = make_int2(r[k], __float_as_int(d[k]));
-              if (nc == 0) c0 = ce;
-              else if (nc == 1) c1 = ce;
-              else if (nc == 2) c2 = ce;
-              else c3 = ce;
-              ++nc;
-            }
-          }
-        } else {
-          const int first = leaf_first(e.x), count = leaf_count(e.x);
-          for (int i = 0; i < count; ++i) {
-            dev::ClosestHit h;
-            h.d2 = FLT_MAX;
-            h.id = INT32_MAX;
-            h.slot = 0;
-            h.cp = p;
-            dev::test_slot(tris, first + i, p, h);
-            const unsigned long long k = hit_key(h.d2, h.id);
-            if (k < my_key) {
-              my_key = k;
-              my_cp = h.cp;
-            }
-          }
-        }
-      }
-      unsigned long long wk = my_key;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) wk = min(wk, __shfl_xor_sync(0xffffffffu, wk, o));
-      best_key = min(best_key, wk);
-      // append this iteration's children (lane order, each lane's nearest last)
-      int incl = nc;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const int total = __shfl_sync(0xffffffffu, incl, 31);
-      int at = sp + incl - nc;
-      const int2 cs[4] = {c0, c1, c2, c3};
-      for (int j = nc - 1; j >= 0; --j, ++at) {
-        if (at < kFinishStack) work[at] = cs[j];
-      }
-      if (sp + total > kFinishStack) dropped = true;
-      sp = min(sp + total, kFinishStack);
-      __syncwarp();
+    dev::WarpBest b;
+    b.key = b.mine = dev::hit_key(out_d2[q], id0 < 0 ? INT32_MAX : id0);
+    b.cp = dev::v3(c0.x, c0.y, c0.z);
+    b.slot = -1;
+    int4 start = make_int4(0, 0, kEmptyChild, kEmptyChild);  // the root
+    if (grid.cells) start = dev::seed_cell(grid, p, 0);
+    dev::warp_search(nodes, tris, p, start, b, work);
+    if (b.winner()) {
+      const int id = static_cast<int>(b.key & 0xffffffffu);
+      out_d2[q] = dev::key_d2(b.key);
+      out_id[q] = id == INT32_MAX ? -1 : id;
+      out_cp[q] = n2w_vec3{b.cp.x, b.cp.y, b.cp.z};
+      out_overflow[q] = b.dropped;
     }
-    // the lane holding the winning key writes it (a triangle is tested by one
-    // lane only); if nothing beat the hand-off bound, the written hit stands
-    if (best_key != start_key && my_key == best_key) {
-      out_d2[q] = __uint_as_float(static_cast<unsigned>(best_key >> 32));
-      out_id[q] = static_cast<int>(best_key & 0xffffffffu);
-      out_cp[q] = n2w_vec3{my_cp.x, my_cp.y, my_cp.z};
-    }
-    if (lane == 0) out_overflow[q] = dropped ? 1 : 0;
     __syncwarp();
+  }
+}
+
+// Small launches: one warp per query (warp_search.cuh).
+template <bool kMasked>
+__global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) closest_point_warp_kernel(
+    const float4* __restrict__ nodes, const float4* __restrict__ tris, const dev::SeedGrid grid,
+    const n2w_vec3* __restrict__ points, const uint8_t* __restrict__ active, int n, float* __restrict__ out_d2,
+    n2w_vec3* __restrict__ out_cp, int* __restrict__ out_id, int* __restrict__ out_overflow) {
+  extern __shared__ int2 s_work[];
+  const int warp = threadIdx.x >> 5;
+  const int q = static_cast<int>(blockIdx.x) * dev::kWarpsPerBlock + warp;
+  if (q >= n) return;
+  const n2w_vec3 pt = points[q];
+  if (kMasked && active[q] == 0) {
+    if ((threadIdx.x & 31) == 0) {
+      out_d2[q] = 0.0f;
+      out_cp[q] = pt;
+      out_id[q] = -1;
+      out_overflow[q] = 0;
+    }
+    return;
+  }
+  const dev::WarpBest b = dev::warp_query(nodes, tris, grid, dev::v3(pt.x, pt.y, pt.z), 0, dev::v3(0.0f, 0.0f, 0.0f),
+                                          s_work + warp * dev::kWarpList);
+  if (b.winner()) {
+    const int id = static_cast<int>(b.key & 0xffffffffu);
+    out_d2[q] = dev::key_d2(b.key);
+    out_cp[q] = n2w_vec3{b.cp.x, b.cp.y, b.cp.z};
+    out_id[q] = id == INT32_MAX ? -1 : id;
+    out_overflow[q] = b.dropped;
   }
 }
 
@@ -374,6 +328,14 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
     N2W_CUDA(cudaGetLastError());
     return;
   }
+  if (n <= kWarpQueries) {
+    const unsigned blocks = static_cast<unsigned>((n + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock);
+    auto kern = d_active ? closest_point_warp_kernel<true> : closest_point_warp_kernel<false>;
+    kern<<<blocks, 32 * dev::kWarpsPerBlock, dev::kWarpSearchBytes, stream>>>(nodes, tris, sg, d_points, d_active, n,
+                                                                             d_d2, d_cp, d_id, d_overflow);
+    N2W_CUDA(cudaGetLastError());
+    return;
+  }
   const bool small = n < kSmallLaunch;
   if (d_active) {
     if (small) launch(closest_point_kernel<true, false, 4>, d_active, nullptr, nullptr);
@@ -383,19 +345,10 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
     else launch(closest_point_kernel<false, false, 5>, nullptr, nullptr, nullptr);
   }
   N2W_CUDA(cudaGetLastError());
-  const size_t smem = sizeof(int2) * kFinishWarps * kFinishStack;
-  static thread_local int configured_device = -1;
-  int dev = 0;
-  N2W_CUDA(cudaGetDevice(&dev));
-  if (configured_device != dev) {
-    N2W_CUDA(cudaFuncSetAttribute(closest_point_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)));
-    configured_device = dev;
-  }
   const int64_t groups = (static_cast<int64_t>(n) + 31) / 32;
-  const unsigned blocks = static_cast<unsigned>((groups + kFinishWarps - 1) / kFinishWarps);
-  closest_point_finish_kernel<<<blocks, 32 * kFinishWarps, smem, stream>>>(nodes, tris, d_points, n, d_d2, d_cp,
-                                                                          d_id, d_overflow);
+  const unsigned blocks = static_cast<unsigned>((groups + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock);
+  closest_point_finish_kernel<<<blocks, 32 * dev::kWarpsPerBlock, dev::kWarpSearchBytes, stream>>>(
+      nodes, tris, sg, d_points, n, d_d2, d_cp, d_id, d_overflow);
   N2W_CUDA(cudaGetLastError());
 }
 

@@ -33,6 +33,7 @@
 #include "philox.cuh"
 #include "problem.cuh"
 #include "walker.cuh"
+#include "warp_search.cuh"
 
 namespace n2w {
 
@@ -500,59 +501,85 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
 }
 
 // ---- per-point first query ----------------------------------------------------
-__global__ void __launch_bounds__(256) first_query_kernel(const float4* __restrict__ nodes,
-                                                          const float4* __restrict__ tris, const dev::SeedGrid grid,
-                                                          const n2w_vec3* __restrict__ points, int64_t n,
-                                                          float4* __restrict__ cpd, int2* __restrict__ ids,
-                                                          n2w_walk_counters* counters) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const n2w_vec3 pt = points[i];
-  const dev::V3 p = dev::v3(pt.x, pt.y, pt.z);
-  dev::ClosestHit hit;
-  hit.d2 = hit.lim = FLT_MAX;
-  hit.id = INT32_MAX;
-  hit.slot = -1;
-  hit.cp = p;
-  dev::TraversalStats st{0, 0, 0};
-  dev::traverse_frames(nodes, tris, grid, p, hit, st, 0);
-  cpd[i] = make_float4(hit.cp.x, hit.cp.y, hit.cp.z, hit.d2);
-  ids[i] = make_int2(hit.id, hit.slot);
-  if (counters) {
-    atomicAdd(&counters->node_visits, static_cast<unsigned long long>(st.node_visits));
-    atomicAdd(&counters->tri_tests, static_cast<unsigned long long>(st.tri_tests));
-    if (st.overflow) atomicAdd(&counters->overflow, 1ull);
+// Point i's place: the mesh's root and grid (batched launches: those of the last
+// instance whose point_base <= i, in the merged scene).
+struct FirstQuery {
+  dev::V3 p;
+  dev::SeedGrid grid;
+  int root;
+};
+template <bool kBatch>
+__device__ __forceinline__ FirstQuery first_query_of(const WalkArgs& a, int64_t i) {
+  FirstQuery f;
+  n2w_vec3 pt;
+  if constexpr (kBatch) {
+    int lo = 0, hi = a.n_insts - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (a.insts[mid].point_base <= i) lo = mid;
+      else hi = mid - 1;
+    }
+    const BatchInst& I = a.insts[lo];
+    pt = I.points[i - I.point_base];
+    f.grid = I.grid;
+    f.root = I.root;
+  } else {
+    pt = a.points[i];
+    f.grid = a.grid;
+    f.root = 0;
   }
+  f.p = dev::v3(pt.x, pt.y, pt.z);
+  return f;
 }
 
-// First queries of a batched launch: point i belongs to the last instance whose
-// point_base <= i; its query starts at that instance's root in the merged scene.
-__global__ void __launch_bounds__(256) first_query_batch_kernel(const __grid_constant__ WalkArgs a, int64_t n,
-                                                                float4* __restrict__ cpd, int2* __restrict__ ids) {
+// One lane per point.
+template <bool kBatch>
+__global__ void __launch_bounds__(256) first_query_kernel(const __grid_constant__ WalkArgs a, int64_t n,
+                                                          float4* __restrict__ cpd, int2* __restrict__ ids) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  int lo = 0, hi = a.n_insts - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (a.insts[mid].point_base <= i) lo = mid;
-    else hi = mid - 1;
-  }
-  const BatchInst& I = a.insts[lo];
-  const n2w_vec3 pt = I.points[i - I.point_base];
-  const dev::V3 p = dev::v3(pt.x, pt.y, pt.z);
+  const FirstQuery f = first_query_of<kBatch>(a, i);
   dev::ClosestHit hit;
   hit.d2 = hit.lim = FLT_MAX;
   hit.id = INT32_MAX;
   hit.slot = -1;
-  hit.cp = p;
+  hit.cp = f.p;
   dev::TraversalStats st{0, 0, 0};
-  dev::traverse_frames(a.nodes, a.tris, I.grid, p, hit, st, I.root);
+  dev::traverse_frames(a.nodes, a.tris, f.grid, f.p, hit, st, f.root);
   cpd[i] = make_float4(hit.cp.x, hit.cp.y, hit.cp.z, hit.d2);
   ids[i] = make_int2(hit.id, hit.slot);
   if (a.counters) {
     atomicAdd(&a.counters->node_visits, static_cast<unsigned long long>(st.node_visits));
     atomicAdd(&a.counters->tri_tests, static_cast<unsigned long long>(st.tri_tests));
     if (st.overflow) atomicAdd(&a.counters->overflow, 1ull);
+  }
+}
+
+// One warp per point (warp_search.cuh): with few points a lane's search is the
+// length of the launch.
+template <bool kBatch>
+__global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) first_query_warp_kernel(const __grid_constant__ WalkArgs a,
+                                                                                    int64_t n,
+                                                                                    float4* __restrict__ cpd,
+                                                                                    int2* __restrict__ ids) {
+  extern __shared__ int2 s_work[];
+  const int warp = threadIdx.x >> 5;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * dev::kWarpsPerBlock + warp;
+  if (i >= n) return;
+  const FirstQuery f = first_query_of<kBatch>(a, i);
+  const dev::WarpBest b =
+      dev::warp_query(a.nodes, a.tris, f.grid, f.p, f.root, f.p, s_work + warp * dev::kWarpList);
+  if (b.winner()) {
+    cpd[i] = make_float4(b.cp.x, b.cp.y, b.cp.z, dev::key_d2(b.key));
+    ids[i] = make_int2(static_cast<int>(b.key & 0xffffffffu), b.slot);
+  }
+  if (a.counters) {
+    const unsigned nodes = __reduce_add_sync(0xffffffffu, b.nodes), tris = __reduce_add_sync(0xffffffffu, b.tris);
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&a.counters->node_visits, static_cast<unsigned long long>(nodes));
+      atomicAdd(&a.counters->tri_tests, static_cast<unsigned long long>(tris));
+      if (b.dropped) atomicAdd(&a.counters->overflow, 1ull);
+    }
   }
 }
 
@@ -633,14 +660,29 @@ void launch_walker(const WalkArgs& a, int block, int blocks_per_sm, cudaStream_t
   N2W_CUDA(cudaGetLastError());
 }
 
+// First queries of n points; up to kWarpPoints points a warp each, else a lane
+// each.  One short walk per point, lane / warp per first query: 294 / 234 us (40
+// points), 370 / 270 (1,000), 458 / 367 (8,000), 481 / 417 (16,000), 567 / 564
+// (32,000).
+constexpr int64_t kWarpPoints = 32768;
+
+template <bool kBatch>
+void launch_first_query(const WalkArgs& a, int64_t n, float4* cpd, int2* ids, cudaStream_t s) {
+  if (n <= kWarpPoints) {
+    const unsigned blocks = static_cast<unsigned>((n + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock);
+    first_query_warp_kernel<kBatch><<<blocks, 32 * dev::kWarpsPerBlock, dev::kWarpSearchBytes, s>>>(a, n, cpd, ids);
+  } else {
+    const int block = 256;
+    first_query_kernel<kBatch><<<static_cast<unsigned>((n + block - 1) / block), block, 0, s>>>(a, n, cpd, ids);
+  }
+  N2W_CUDA(cudaGetLastError());
+}
+
 }  // namespace
 
 void launch_first_query_batch(const WalkArgs& a, int64_t total_points, float4* cpd, int2* ids, cudaStream_t s) {
   if (total_points == 0) return;
-  const int block = 256;
-  first_query_batch_kernel<<<static_cast<unsigned>((total_points + block - 1) / block), block, 0, s>>>(
-      a, total_points, cpd, ids);
-  N2W_CUDA(cudaGetLastError());
+  launch_first_query<true>(a, total_points, cpd, ids, s);
 }
 
 // Two register budgets for the batched walker: 64 registers (4 resident
@@ -744,13 +786,7 @@ void run_walker(WalkArgs& a, int64_t point_count, int out_kind, int walk_mode, c
   int2* ids = reinterpret_cast<int2*>(base + kWsHeader + 16 * static_cast<size_t>(point_count));
   a.first_cpd = cpd;
   a.first_ids = ids;
-  {
-    const int block = 256;
-    const int64_t grid = (point_count + block - 1) / block;
-    first_query_kernel<<<static_cast<unsigned>(grid), block, 0, stream>>>(a.nodes, a.tris, a.grid, a.points,
-                                                                          point_count, cpd, ids, a.counters);
-    N2W_CUDA(cudaGetLastError());
-  }
+  launch_first_query<false>(a, point_count, cpd, ids, stream);
   const int block = o.block_size > 0 ? o.block_size : kDefaultWalkerThreads;
   if (out_kind == kOutStats) launch_walker<kOutStats, N2W_WALK_PURE>(a, block, o.blocks_per_sm, stream);
   else if (out_kind == kOutSamples) launch_walker<kOutSamples, N2W_WALK_PURE>(a, block, o.blocks_per_sm, stream);
