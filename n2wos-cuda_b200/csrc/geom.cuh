@@ -192,11 +192,19 @@ __device__ __forceinline__ void cswap(float& da, int& ra, float& db, int& rb) {
 // the lanes' lists.  262,144 / 4,194,304 uniform queries 391 -> 374 us / 4.77 ->
 // 4.37 ms, Laplace / Poisson walks 17.4 -> 16.0 / 46.1 -> 43.4 ms, batched
 // instances 37.3 -> 33.8 ms (evict_first: 17.1 / 45.0 / 36.4; evict_last: as
-// without a hint).
+// without a hint).  kL1 keeps the allocation for launches of few walkers per
+// SM, whose nodes do fit.
+template <bool kL1 = false>
 __device__ __forceinline__ void ldg_v8f(const float4* p, float4& a, float4& b) {
-  asm("ld.global.nc.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-      : "l"(p));
+  if constexpr (kL1) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+  } else {
+    asm("ld.global.nc.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+  }
 }
 __device__ __forceinline__ int4 ldg_v8_first_int4(const float4* p) {
   int4 a;
@@ -217,15 +225,16 @@ __device__ __forceinline__ void load_node(const float4* __restrict__ nodes, int3
 }
 
 // load_node of a FrameNode4: the last load also brings the node's frame v.
+template <bool kL1 = false>
 __device__ __forceinline__ void load_frame_node(const float4* __restrict__ frames, int32_t ref, float4& lox,
                                                 float4& hix, float4& loy, float4& hiy, float4& loz, float4& hiz,
                                                 int4& ch, V3& v) {
   const float4* n = frames + static_cast<size_t>(ref) * 8;
   float4 c, f;
-  ldg_v8f(n + 0, lox, hix);
-  ldg_v8f(n + 2, loy, hiy);
-  ldg_v8f(n + 4, loz, hiz);
-  ldg_v8f(n + 6, c, f);
+  ldg_v8f<kL1>(n + 0, lox, hix);
+  ldg_v8f<kL1>(n + 2, loy, hiy);
+  ldg_v8f<kL1>(n + 4, loz, hiz);
+  ldg_v8f<kL1>(n + 6, c, f);
   ch = make_int4(__float_as_int(c.x), __float_as_int(c.y), __float_as_int(c.z), __float_as_int(c.w));
   v = v3(f.x, f.y, f.z);
 }
@@ -262,12 +271,12 @@ struct ClosestHit {
 // (d2, id) order.  Seeding a query with real candidates gives the traversal a
 // tight bound without changing its answer.  kFast selects the contracted-FP32
 // triangle routine (walker); callers use the test_slot / test_slot_fast wrappers.
-template <bool kFast>
+template <bool kFast, bool kL1 = false>
 __device__ __forceinline__ void test_slot_impl(const float4* __restrict__ tris, int slot, V3 p, ClosestHit& hit) {
   const float4* t = tris + static_cast<size_t>(slot) * 4;
   float4 r0, r1, r2, r3;
-  ldg_v8f(t + 0, r0, r1);
-  ldg_v8f(t + 2, r2, r3);
+  ldg_v8f<kL1>(t + 0, r0, r1);
+  ldg_v8f<kL1>(t + 2, r2, r3);
   const V3 a = v3(r0.x, r0.y, r0.z), ab = v3(r1.x, r1.y, r1.z), ac = v3(r1.w, r2.x, r2.y),
            b = v3(r2.z, r2.w, r3.x), c = v3(r3.y, r3.z, r3.w);
   V3 cp;
@@ -294,8 +303,9 @@ __device__ __forceinline__ void test_slot_impl(const float4* __restrict__ tris, 
 __device__ __forceinline__ void test_slot(const float4* __restrict__ tris, int slot, V3 p, ClosestHit& hit) {
   test_slot_impl<false>(tris, slot, p, hit);
 }
+template <bool kL1>
 __device__ __forceinline__ void test_slot_fast(const float4* __restrict__ tris, int slot, V3 p, ClosestHit& hit) {
-  test_slot_impl<true>(tris, slot, p, hit);
+  test_slot_impl<true, kL1>(tris, slot, p, hit);
 }
 
 // Seed grid: (n+1)^3 lattice nodes over a padded mesh box.  A node's cell {x: the
@@ -526,7 +536,7 @@ struct FrameStack {
 
 // Tests one pending triangle, if there is one.  The current best is not tested
 // again (queries start with it tested as a seed).
-template <bool kFast>
+template <bool kFast, bool kL1 = false>
 __device__ __forceinline__ void trav_triangle(const float4* __restrict__ tris, V3 p, ClosestHit& hit, FrameTrav& t,
                                               FrameStack& st, uint32_t& c_tris) {
   if (t.leaf_cur >= t.leaf_end && t.lp > 0) {
@@ -536,7 +546,7 @@ __device__ __forceinline__ void trav_triangle(const float4* __restrict__ tris, V
   }
   if (t.leaf_cur < t.leaf_end) {
     if (t.leaf_cur != hit.slot) {
-      test_slot_impl<kFast>(tris, t.leaf_cur, p, hit);
+      test_slot_impl<kFast, kL1>(tris, t.leaf_cur, p, hit);
       ++c_tris;
     }
     ++t.leaf_cur;
@@ -546,6 +556,7 @@ __device__ __forceinline__ void trav_triangle(const float4* __restrict__ tris, V
 // Expands one pending node, if there is one and the leaf list has room.  The
 // children within the limit go to the lists by predicated stores (branches per
 // child left 9 of 32 lanes active), the last inner one is entered.
+template <bool kL1 = false>
 __device__ __forceinline__ void trav_node(const float4* __restrict__ frames, V3 p, const ClosestHit& hit, FrameTrav& t,
                                           FrameStack& st, uint32_t& c_nodes, bool& overflow) {
   if (t.ref == kEmptyChild && t.np > 0) t.ref = st.nodes[--t.np];
@@ -553,7 +564,7 @@ __device__ __forceinline__ void trav_node(const float4* __restrict__ frames, V3 
     float4 lox, hix, loy, hiy, loz, hiz;
     int4 ch;
     V3 v;
-    load_frame_node(frames, t.ref, lox, hix, loy, hiy, loz, hiz, ch, v);
+    load_frame_node<kL1>(frames, t.ref, lox, hix, loy, hiy, loz, hiz, ch, v);
     ++c_nodes;
     const V3 q = to_frame(v, p);
     const bool k0 = box_d2_fast(q, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x) <= hit.lim;

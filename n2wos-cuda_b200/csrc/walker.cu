@@ -193,7 +193,7 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 //    warp returns to Phase A once `regen` lanes are waiting (or none is busy),
 //    so the walk updates run for many lanes at once and no lane waits for
 //    another lane's whole traversal.
-template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks>
+template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks, bool kL1 = false>
 __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(const __grid_constant__ WalkArgs a) {
   static_assert(!kBatch || (kOut == kOutStats && kWalk == N2W_WALK_PURE),
                 "batched launches run plain walks into per-point statistics");
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
 
   bool alive = false;     // a walk is in progress on this lane
   bool querying = false;  // its closest-point query is in flight
-  bool exhausted = false; // the global queue has no chunk left for this lane
+  bool exhausted = lane >= a.lanes;  // the global queue has no chunk left for this lane
   int64_t pid = -1;  // global point index
   int inst = 0;      // batched launches: instance of the current chunk
   int walk = 0, walk_end = 0;
@@ -448,10 +448,10 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
         if constexpr (kBatch) root = a.insts[inst].root;
         int4 cell = make_int4(prev_slot, root, kEmptyChild, kEmptyChild);
         if (grid.cells) cell = dev::seed_cell(grid, x, root);
-        dev::test_slot_fast(a.tris, prev_slot, x, hit);
+        dev::test_slot_fast<kL1>(a.tris, prev_slot, x, hit);
         ++c_tris;
         if (cell.x != prev_slot) {
-          dev::test_slot_fast(a.tris, cell.x, x, hit);
+          dev::test_slot_fast<kL1>(a.tris, cell.x, x, hit);
           ++c_tris;
         }
         tv.start(cell, stack);
@@ -466,8 +466,8 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
       if (busy == 0 || __popc(waiting) >= a.regen) break;
       if (querying) {
         bool ov = false;
-        dev::trav_triangle<true>(a.tris, x, hit, tv, stack, c_tris);
-        dev::trav_node(a.nodes, x, hit, tv, stack, c_nodes, ov);
+        dev::trav_triangle<true, kL1>(a.tris, x, hit, tv, stack, c_tris);
+        dev::trav_node<kL1>(a.nodes, x, hit, tv, stack, c_nodes, ov);
         querying = !tv.done();
         if (ov) {
           w_overflow = true;
@@ -645,19 +645,44 @@ __global__ void combine_kernel(const float* __restrict__ cache, const float* __r
 // ---- host side -----------------------------------------------------------
 namespace {
 
-template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks>
-void launch_walker(const WalkArgs& a, int block, int blocks_per_sm, cudaStream_t stream) {
-  auto kern = walker_kernel<kOut, kWalk, kBatch, kMinBlocks>;
+// Launches of few walks: as many warps as kSpreadWarps per SM share them, each
+// with as few lanes as that takes, so a walk's serial chain of queries does not
+// wait for its warp's other lanes and all SMs work; nodes stay in L1 there (with
+// L1 bypassed 889 us for the first figure).  37 points x 64 walks 1,205 -> 692 us,
+// 10 / 300 / 1,000 / 2,000 points x 16 walks 1,310 / 2,237 / 2,239 / 2,405 -> 736 /
+// 1,653 / 1,829 / 2,129 us; 4 / 8 / 32 / 64 warps per SM: 728 / 696 / 692 / 691 us
+// and 2,408 / 2,173 / 2,238 / 2,447 us for the first and the last.
+constexpr int kSpreadWarps = 16;
+
+template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks, bool kL1 = false>
+void launch_walker_kernel(WalkArgs a, int block, int blocks_per_sm, cudaStream_t stream) {
+  auto kern = walker_kernel<kOut, kWalk, kBatch, kMinBlocks, kL1>;
   int occ = 0;
   N2W_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, block, 0));
   if (occ < 1) occ = 1;
   const int per_sm = blocks_per_sm > 0 ? std::min(blocks_per_sm, occ) : occ;
-  const int64_t lanes_needed = a.total_chunks;
-  int64_t grid = static_cast<int64_t>(sm_count_current()) * per_sm;
-  grid = std::min<int64_t>(grid, (lanes_needed + block - 1) / block);
+  const int64_t sms = sm_count_current();
+  int64_t grid = sms * per_sm;
+  const int64_t per_block = static_cast<int64_t>(block / 32) * a.lanes;
+  grid = std::min<int64_t>(grid, (a.total_chunks + per_block - 1) / per_block);
   grid = std::max<int64_t>(grid, 1);
   kern<<<static_cast<unsigned>(grid), block, 0, stream>>>(a);
   N2W_CUDA(cudaGetLastError());
+}
+
+template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks>
+void launch_walker(WalkArgs a, int block, int blocks_per_sm, cudaStream_t stream) {
+  a.lanes = 32;
+  if constexpr (!kBatch) {
+    const int64_t warps = static_cast<int64_t>(sm_count_current()) * kSpreadWarps;
+    const int64_t lanes = (a.total_chunks + warps - 1) / warps;
+    if (lanes < 32) {
+      a.lanes = static_cast<int>(lanes);
+      a.regen = std::max(1, a.regen * a.lanes / 32);
+      return launch_walker_kernel<kOut, kWalk, kBatch, kMinBlocks, true>(a, block, blocks_per_sm, stream);
+    }
+  }
+  launch_walker_kernel<kOut, kWalk, kBatch, kMinBlocks>(a, block, blocks_per_sm, stream);
 }
 
 // First queries of n points; up to kWarpPoints points a warp each, else a lane

@@ -74,6 +74,7 @@ struct WalkArgs {
   int walks_per_point;
   int chunk;
   int regen;  // waiting lanes that trigger the walk-update phase
+  int lanes;  // lanes of a warp that take walks
   int max_steps;
   int depth_m;
   float eps;
