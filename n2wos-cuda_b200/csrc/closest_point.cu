@@ -30,7 +30,7 @@ dev::SeedGrid seed_grid_of(const n2w_bvh& b) {
 namespace {
 
 // Persistent state machine, one lane per query.  Every iteration each busy
-// lane advances its query by one step (dev::trav_triangle + dev::trav_node; the
+// lane advances its query by one step (a triangle and two nodes; the
 // counting variant by one unit of dev::trav_step_boxes), and a lane whose query
 // is complete writes it and takes the next query in the same iteration.  Each
 // block owns the contiguous range [b n / B, (b + 1) n / B) of the queries and
@@ -48,9 +48,10 @@ constexpr int kQueryBlock = 256;
 // thousands against a mean of ~40, and one of them per lane would set the
 // launch's length.  With more queries per lane the lanes' totals even out and
 // the budget grows in proportion, so a full GPU hands off only the extreme
-// queries.  262,144 uniform queries: 399 / 392 / 423 / 451 / 481 us with a
-// budget of 96 / 128 / 192 / 256 / 384; 4,194,304: 4.78 ms with any of them.
-constexpr uint32_t kQueryBudget = 128;
+// queries.  Budget 64 / 80 / 96 / 112 / 128: 409 / 370 / 357 / 357 / 362 us
+// (262,144 uniform queries), 179 / 181 / 183 / 187 / 190 us (300,000 near the
+// surface), 170 / 153 / 158 / 151 / 151 us (40,000); 4,194,304: the same.
+constexpr uint32_t kQueryBudget = 112;
 constexpr int kHandOff = 2;         // overflow-slot mark of a handed-off query
 // Launches of at most this many queries give each query a warp: with a lane per
 // query a launch lasts as long as its slowest serial search, whatever its size.
@@ -58,12 +59,10 @@ constexpr int kHandOff = 2;         // overflow-slot mark of a handed-off query
 // queries), 126 / 12 (1,000), 144 / 26 (4,000), 151 / 74 (16,000), 153 / 141
 // (32,000), 374 / 1,076 (262,144).
 constexpr int kWarpQueries = 32768;
-// Resident blocks per SM the traversal is compiled for (kMinBlocks).  Launches
-// of up to a few queries per lane run faster with 4 (up to 64 registers, no
-// spills) and larger ones with 5 (more warps to hide load latency): measured
-// 152.5 / 224.2 / 285.1 against 149.5 / 213.0 / 276.0 M queries/s at 131,072 /
-// 262,144 / 524,288 queries, equal at 1 M and 2 M, 391 against 405 at 4 M.
-constexpr int64_t kSmallLaunch = int64_t{1} << 21;
+// Resident blocks per SM the traversal is compiled for: 4 (56-62 registers, no
+// spills).  3 / 4 / 5: 420 / 372 / 404 us (262,144 uniform queries), 426 / 423 / 503
+// us (1,000,003 masked, near the surface), 4.38 / 4.22 / 4.37 ms (4,194,304).
+constexpr int kQueryBlocks = 4;
 
 // One lane's query in flight; step() returns false once it is complete.
 template <bool kCount>
@@ -73,7 +72,11 @@ struct Search {
   __device__ __forceinline__ void start(int4 cell) { t.start(cell, stack); }
   __device__ __forceinline__ bool step(const float4* __restrict__ frames, const float4* __restrict__ tris, dev::V3 p,
                                        dev::ClosestHit& hit, uint32_t& c_nodes, uint32_t& c_tris, bool& overflow) {
+    // Two nodes per triangle: uniform queries expand 26 nodes and test 13
+    // triangles (one node: 372 against 357 us for 262,144 queries, equal for
+    // 1,000,003 near the surface and 4,194,304).
     dev::trav_triangle<false>(tris, p, hit, t, stack, c_tris);
+    dev::trav_node(frames, p, hit, t, stack, c_nodes, overflow);
     dev::trav_node(frames, p, hit, t, stack, c_nodes, overflow);
     return !t.done();
   }
@@ -89,8 +92,8 @@ struct Search<true> {
   }
 };
 
-template <bool kMasked, bool kCount, int kMinBlocks>
-__global__ void __launch_bounds__(kQueryBlock, kMinBlocks) closest_point_kernel(
+template <bool kMasked, bool kCount>
+__global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kernel(
     const float4* __restrict__ nodes, const float4* __restrict__ tris, const dev::SeedGrid grid,
     const n2w_vec3* __restrict__ points, const uint8_t* __restrict__ active, int n,
     float* __restrict__ out_d2, n2w_vec3* __restrict__ out_cp, int* __restrict__ out_id,
@@ -324,7 +327,7 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
   if (d_nodes) {
     // the counting variant runs every query to completion in one lane, so its
     // counts are the single-lane traversal's (the algorithmic work)
-    launch(closest_point_kernel<false, true, 5>, d_active, d_nodes, d_tris);
+    launch(closest_point_kernel<false, true>, d_active, d_nodes, d_tris);
     N2W_CUDA(cudaGetLastError());
     return;
   }
@@ -336,14 +339,8 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
     N2W_CUDA(cudaGetLastError());
     return;
   }
-  const bool small = n < kSmallLaunch;
-  if (d_active) {
-    if (small) launch(closest_point_kernel<true, false, 4>, d_active, nullptr, nullptr);
-    else launch(closest_point_kernel<true, false, 5>, d_active, nullptr, nullptr);
-  } else {
-    if (small) launch(closest_point_kernel<false, false, 4>, nullptr, nullptr, nullptr);
-    else launch(closest_point_kernel<false, false, 5>, nullptr, nullptr, nullptr);
-  }
+  if (d_active) launch(closest_point_kernel<true, false>, d_active, nullptr, nullptr);
+  else launch(closest_point_kernel<false, false>, nullptr, nullptr, nullptr);
   N2W_CUDA(cudaGetLastError());
   const int64_t groups = (static_cast<int64_t>(n) + 31) / 32;
   const unsigned blocks = static_cast<unsigned>((groups + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock);
