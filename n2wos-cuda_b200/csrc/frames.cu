@@ -78,7 +78,8 @@ __device__ __forceinline__ bool mirror_onto(dev::V3 n, int c, dev::V3& v) {
   const float l2 = w.x * w.x + w.y * w.y + w.z * w.z;
   if (!(l2 > 1.0e-8f)) return false;
   const float s = sqrtf(2.0f / l2);
-  v = dev::v3(w.x * s, w.y * s, w.z * s);
+  const float sign = w.z < 0.0f ? -s : s;  // v and -v are the same mirror
+  v = dev::frame_v(w.x * sign, w.y * sign);
   return true;
 }
 
@@ -91,8 +92,7 @@ __global__ void __launch_bounds__(kFrameBlock) frame_nodes_kernel(const Node4* _
   if (node >= n) return;
   const Node4& nd = nodes[node];
   const TriRange r = ranges[node];
-  dev::V3 v = dev::v3(0.0f, 0.0f, 0.0f);
-  bool framed = false;
+  dev::V3 v = dev::frame_v(0.0f, 0.0f);  // the axes, z mirrored
   float pad = 0.0f;
   int first[4], last[4];
   for (int k = 0; k < 4; ++k) {
@@ -100,7 +100,9 @@ __global__ void __launch_bounds__(kFrameBlock) frame_nodes_kernel(const Node4* _
     first[k] = c == kEmptyChild ? 0 : (c >= 0 ? ranges[c].first : leaf_first(c));
     last[k] = c == kEmptyChild ? 0 : (c >= 0 ? ranges[c].last : leaf_first(c) + leaf_count(c));
   }
-  if (r.last - r.first <= kFrameMaxTris) {
+  float lo[4][3], hi[4][3];
+  const bool small = r.last - r.first <= kFrameMaxTris;
+  if (small) {
     float nx = 0.0f, ny = 0.0f, nz = 0.0f, big = 0.0f;
     for (int t = r.first + lane; t < r.last; t += 32) {
       const dev::V3 a = vertex(tris, t, 0), b = vertex(tris, t, 1), c = vertex(tris, t, 2);
@@ -114,55 +116,79 @@ __global__ void __launch_bounds__(kFrameBlock) frame_nodes_kernel(const Node4* _
     nx = warp_sum(nx);
     ny = warp_sum(ny);
     nz = warp_sum(nz);
-    // 2^-19 of the largest |vertex|_1: 7 u of the frame's rounding plus the
-    // closest-point arithmetic's few u, twice over (u = 2^-24)
-    pad = warp_max(big) * 1.9073486328125e-06f + 1e-30f;
+    pad = warp_max(big);
     const float len = sqrtf(nx * nx + ny * ny + nz * nz);
     const dev::V3 nrm = dev::v3(nx / len, ny / len, nz / len);
     float best = INFINITY;
     for (int c = 0; c < kFrameCandidates; ++c) {
-      dev::V3 w = dev::v3(0.0f, 0.0f, 0.0f);
+      dev::V3 w = dev::frame_v(0.0f, 0.0f);
       if (c > 0 && (!(len > 0.0f) || !mirror_onto(nrm, c, w))) continue;
       float cost = 0.0f;
       for (int k = 0; k < 4; ++k) {
         if (first[k] >= last[k]) continue;
-        float lo[3], hi[3];
-        frame_bounds(tris, first[k], last[k], w, lo, hi);
-        const float ex = hi[0] - lo[0], ey = hi[1] - lo[1], ez = hi[2] - lo[2];
+        frame_bounds(tris, first[k], last[k], w, lo[k], hi[k]);
+        const float ex = hi[k][0] - lo[k][0], ey = hi[k][1] - lo[k][1], ez = hi[k][2] - lo[k][2];
         cost += ex * ey + ey * ez + ez * ex;
       }
       if (cost < 0.98f * best) {  // the axes stand unless a frame is clearly better
         best = cost;
         v = w;
-        framed = c > 0;
       }
     }
-  }
-  FrameNode4 o;
-  for (int k = 0; k < 4; ++k) {
-    o.child[k] = nd.child[k];
-    if (framed && nd.child[k] != kEmptyChild) {
-      float lo[3], hi[3];
-      frame_bounds(tris, first[k], last[k], v, lo, hi);
-      o.lo_x[k] = lo[0] - pad;
-      o.hi_x[k] = hi[0] + pad;
-      o.lo_y[k] = lo[1] - pad;
-      o.hi_y[k] = hi[1] + pad;
-      o.lo_z[k] = lo[2] - pad;
-      o.hi_z[k] = hi[2] + pad;
-    } else {
-      o.lo_x[k] = nd.lo_x[k];
-      o.hi_x[k] = nd.hi_x[k];
-      o.lo_y[k] = nd.lo_y[k];
-      o.hi_y[k] = nd.hi_y[k];
-      o.lo_z[k] = nd.lo_z[k];
-      o.hi_z[k] = nd.hi_z[k];
+    for (int k = 0; k < 4; ++k) {
+      if (first[k] < last[k]) frame_bounds(tris, first[k], last[k], v, lo[k], hi[k]);
+    }
+  } else {
+    // the boxes that the node has, z mirrored
+    for (int k = 0; k < 4; ++k) {
+      lo[k][0] = nd.lo_x[k];
+      hi[k][0] = nd.hi_x[k];
+      lo[k][1] = nd.lo_y[k];
+      hi[k][1] = nd.hi_y[k];
+      lo[k][2] = -nd.hi_z[k];
+      hi[k][2] = -nd.lo_z[k];
+      if (nd.child[k] == kEmptyChild) continue;
+      for (int a = 0; a < 3; ++a) pad = fmaxf(pad, 3.0f * fmaxf(fabsf(lo[k][a]), fabsf(hi[k][a])));
     }
   }
-  o.v[0] = v.x;
-  o.v[1] = v.y;
-  o.v[2] = v.z;
-  o.pad = 0;
+  // 2^-19 of the largest |vertex|_1: 8 u of the frame's rounding plus the
+  // closest-point arithmetic's few u, twice over (u = 2^-24)
+  const float big1 = pad;
+  pad = pad * 1.9073486328125e-06f + 1e-30f;
+  FrameNode4 o;
+  o.vx = v.x;
+  o.vy = v.y;
+  o.exps = 0;
+  for (int a = 0; a < 3; ++a) {
+    float omin = INFINITY, omax = -INFINITY;
+    for (int k = 0; k < 4; ++k) {
+      if (nd.child[k] == kEmptyChild) continue;
+      omin = fminf(omin, lo[k][a] - pad);
+      omax = fmaxf(omax, hi[k][a] + pad);
+    }
+    // The step: a power of two with the children within 253 of them, at least
+    // 2^-20 of the coordinates so the origin's rounding is a fraction of it.
+    const float want = fmaxf((omax - omin) / 253.0f, fmaxf(big1 * 9.5367431640625e-07f, 1.0e-35f));
+    int e = 0;
+    frexpf(want, &e);  // want <= 2^e
+    e = min(max(e, -120), 120);
+    const float step = ldexpf(1.0f, e);
+    const float origin = omin - step;
+    o.o[a] = origin;
+    o.exps |= static_cast<uint32_t>(e + 127) << (8 * a);
+    uint32_t wl = 0, wh = 0;
+    for (int k = 0; k < 4; ++k) {
+      if (nd.child[k] == kEmptyChild) continue;
+      // outwards by a quarter of a step, for the origin's and the quotient's rounding
+      const float bl = floorf((lo[k][a] - pad - origin) / step - 0.25f);
+      const float bh = ceilf((hi[k][a] + pad - origin) / step + 0.25f);
+      wl |= static_cast<uint32_t>(fminf(fmaxf(bl, 0.0f), 255.0f)) << (8 * k);
+      wh |= static_cast<uint32_t>(fminf(fmaxf(bh, 0.0f), 255.0f)) << (8 * k);
+    }
+    o.plane[2 * a] = wl;
+    o.plane[2 * a + 1] = wh;
+  }
+  for (int k = 0; k < 4; ++k) o.child[k] = nd.child[k];
   if (lane == 0) out[node] = o;
 }
 
@@ -206,24 +232,26 @@ __global__ void __launch_bounds__(256) cell_entries_kernel(const float4* __restr
       changed = false;
       for (int j = 0; j < count; ++j) {
         if (e[j] < 0) continue;
-        float4 lx, hx, ly, hy, lz, hz;
-        int4 ch;
-        dev::V3 v;
-        dev::load_frame_node(frames, e[j], lx, hx, ly, hy, lz, hz, ch, v);
-        const dev::V3 q = dev::to_frame(v, c);
+        const dev::FrameData f = dev::load_frame_node(frames, e[j]);
+        const dev::V3 v = f.v, m = dev::to_frame(v, c);
+        const float q[3] = {m.x - f.o.x, m.y - f.o.y, m.z - f.o.z};
         // half extents of the cube in the frame
-        const float ex = half * (fabsf(1.0f - v.x * v.x) + fabsf(v.x * v.y) + fabsf(v.x * v.z));
-        const float ey = half * (fabsf(v.y * v.x) + fabsf(1.0f - v.y * v.y) + fabsf(v.y * v.z));
-        const float ez = half * (fabsf(v.z * v.x) + fabsf(v.z * v.y) + fabsf(1.0f - v.z * v.z));
-        const float lo[4][3] = {{lx.x, ly.x, lz.x}, {lx.y, ly.y, lz.y}, {lx.z, ly.z, lz.z}, {lx.w, ly.w, lz.w}};
-        const float hi[4][3] = {{hx.x, hy.x, hz.x}, {hx.y, hy.y, hz.y}, {hx.z, hy.z, hz.z}, {hx.w, hy.w, hz.w}};
-        const int kids[4] = {ch.x, ch.y, ch.z, ch.w};
+        const float ext[3] = {half * (fabsf(1.0f - v.x * v.x) + fabsf(v.x * v.y) + fabsf(v.x * v.z)),
+                              half * (fabsf(v.y * v.x) + fabsf(1.0f - v.y * v.y) + fabsf(v.y * v.z)),
+                              half * (fabsf(v.z * v.x) + fabsf(v.z * v.y) + fabsf(1.0f - v.z * v.z))};
+        const int kids[4] = {f.ch.x, f.ch.y, f.ch.z, f.ch.w};
         int keep[4], nk = 0;
         for (int k = 0; k < 4; ++k) {
           if (kids[k] == kEmptyChild) continue;
-          const float dc = dev::box_d2_fast(q, lo[k][0], hi[k][0], lo[k][1], hi[k][1], lo[k][2], hi[k][2]);
-          const float dq = dev::box_d2_fast(q, lo[k][0] - ex, hi[k][0] + ex, lo[k][1] - ey, hi[k][1] + ey,
-                                            lo[k][2] - ez, hi[k][2] + ez);
+          float dc = 0.0f, dq = 0.0f;
+          for (int a = 0; a < 3; ++a) {
+            const float l = f.step[a] * static_cast<float>((f.plane[2 * a] >> (8 * k)) & 255u);
+            const float u = f.step[a] * static_cast<float>((f.plane[2 * a + 1] >> (8 * k)) & 255u);
+            const float gc = q[a] - fminf(fmaxf(q[a], l), u);
+            const float gq = q[a] - fminf(fmaxf(q[a], l - ext[a]), u + ext[a]);
+            dc += gc * gc;
+            dq += gq * gq;
+          }
           if (dc <= lim_c && dq <= lim_q) keep[nk++] = kids[k];
         }
         if (nk == 0 || count - 1 + nk > dev::kCellEntries) continue;

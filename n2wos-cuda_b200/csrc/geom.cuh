@@ -224,39 +224,131 @@ __device__ __forceinline__ void load_node(const float4* __restrict__ nodes, int3
   ch = ldg_v8_first_int4(n + 6);
 }
 
-// load_node of a FrameNode4: the last load also brings the node's frame v.
-template <bool kL1 = false>
-__device__ __forceinline__ void load_frame_node(const float4* __restrict__ frames, int32_t ref, float4& lox,
-                                                float4& hix, float4& loy, float4& hiy, float4& loz, float4& hiz,
-                                                int4& ch, V3& v) {
-  const float4* n = frames + static_cast<size_t>(ref) * 8;
-  float4 c, f;
-  ldg_v8f<kL1>(n + 0, lox, hix);
-  ldg_v8f<kL1>(n + 2, loy, hiy);
-  ldg_v8f<kL1>(n + 4, loz, hiz);
-  ldg_v8f<kL1>(n + 6, c, f);
-  ch = make_int4(__float_as_int(c.x), __float_as_int(c.y), __float_as_int(c.z), __float_as_int(c.w));
-  v = v3(f.x, f.y, f.z);
+struct Rec64 {  // a 64-byte record as loaded
+  float4 r0, r1, r2, r3;
+};
+template <bool kL1>
+__device__ __forceinline__ Rec64 load_rec(const float4* __restrict__ base, int index) {
+  const float4* t = base + static_cast<size_t>(index) * 4;
+  Rec64 r;
+  ldg_v8f<kL1>(t + 0, r.r0, r.r1);
+  ldg_v8f<kL1>(t + 2, r.r2, r.r3);
+  return r;
 }
 
-// p in the frame of a node (layout.h): p - v (v.p).
+// ---- frame nodes (layout.h FrameNode4) ------------------------------------------
+// The mirror of a node's frame; v.z from |v|^2 = 2 (off by at most 2^-22 v.z).
+__device__ __forceinline__ V3 frame_v(float x, float y) {
+  float z;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(z) : "f"(fmaxf(fmaf(-x, x, fmaf(-y, y, 2.0f)), 0.0f)));
+  return v3(x, y, z);
+}
+
+// p in the frame: p - v (v.p).
 __device__ __forceinline__ V3 to_frame(V3 v, V3 p) {
   const float s = fmaf(v.z, p.z, fmaf(v.y, p.y, v.x * p.x));
   return V3{fmaf(-s, v.x, p.x), fmaf(-s, v.y, p.y), fmaf(-s, v.z, p.z)};
 }
 
+struct FrameData {
+  V3 v, o;
+  float step[3];      // 2^e of each axis
+  uint32_t plane[6];
+  int4 ch;
+};
+__device__ __forceinline__ FrameData decode_frame_node(const Rec64& r) {
+  const float4 a = r.r0, b = r.r1, c = r.r2, d = r.r3;
+  FrameData f;
+  f.v = frame_v(a.x, a.y);
+  f.o = v3(a.z, a.w, b.x);
+  const uint32_t e = __float_as_uint(b.y);
+  f.step[0] = __uint_as_float((e << 23) & 0x7f800000u);
+  f.step[1] = __uint_as_float((e << 15) & 0x7f800000u);
+  f.step[2] = __uint_as_float((e << 7) & 0x7f800000u);
+  f.plane[0] = __float_as_uint(b.z);
+  f.plane[1] = __float_as_uint(b.w);
+  f.plane[2] = __float_as_uint(c.x);
+  f.plane[3] = __float_as_uint(c.y);
+  f.plane[4] = __float_as_uint(c.z);
+  f.plane[5] = __float_as_uint(c.w);
+  f.ch = make_int4(__float_as_int(d.x), __float_as_int(d.y), __float_as_int(d.z), __float_as_int(d.w));
+  return f;
+}
+
+template <bool kL1 = false>
+__device__ __forceinline__ FrameData load_frame_node(const float4* __restrict__ frames, int32_t ref) {
+  return decode_frame_node(load_rec<kL1>(frames, ref));
+}
+
+// 32768 + byte k of w: the byte's bits in the mantissa.
+template <int k>
+__device__ __forceinline__ float plane_bits(uint32_t w) {
+  return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7404u + (k << 4)));
+}
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// The largest of a, b and 0; NaN if one is.
+__device__ __forceinline__ float max3_0(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2, 0f00000000;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
+// Adds one axis's squared gaps between q (relative to o) and the boxes of
+// children k, k + 1: max(lo - q, q - hi, 0) with the planes (32768 + b) 2^e -
+// 32768 2^e folded into the subtractions (near = -32768 2^e - q, rounded by at
+// most 2^-9 of a step or u |q|; far = -near).
+template <int k>
+__device__ __forceinline__ uint64_t add_gap2(uint64_t d, uint32_t wlo, uint32_t whi, uint64_t step, uint64_t neg_step,
+                                             uint64_t near, uint64_t far) {
+  float l0, l1, h0, h1;
+  unpack2(fma2(pack2(plane_bits<k>(wlo), plane_bits<k + 1>(wlo)), step, near), l0, l1);
+  unpack2(fma2(pack2(plane_bits<k>(whi), plane_bits<k + 1>(whi)), neg_step, far), h0, h1);
+  const uint64_t g = pack2(max3_0(l0, h0), max3_0(l1, h1));
+  return fma2(g, g, d);
+}
+
+// Squared distances from p to the four child boxes of a node (two children per
+// instruction where there is a packed form; slots without a child: any number).
+__device__ __forceinline__ void frame_distances(const FrameData& f, V3 p, float (&d)[4]) {
+  const V3 m = to_frame(f.v, p);
+  const float q[3] = {m.x - f.o.x, m.y - f.o.y, m.z - f.o.z};
+  uint64_t d01 = 0, d23 = 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float s = f.step[a], nr = fmaf(-32768.0f, s, -q[a]);
+    const uint64_t step = pack2(s, s), neg_step = pack2(-s, -s), near = pack2(nr, nr), far = pack2(-nr, -nr);
+    d01 = add_gap2<0>(d01, f.plane[2 * a], f.plane[2 * a + 1], step, neg_step, near, far);
+    d23 = add_gap2<2>(d23, f.plane[2 * a], f.plane[2 * a + 1], step, neg_step, near, far);
+  }
+  unpack2(d01, d[0], d[1]);
+  unpack2(d23, d[2], d[3]);
+}
+
+__device__ __forceinline__ bool is_leaf(int c) { return static_cast<int>(0u - static_cast<unsigned>(c)) > 0; }
+
 // Largest computed box distance^2, in a node's frame, that a box holding a
 // triangle at computed distance^2 `best` can have.  With u = 2^-24 the frame's
-// coordinates of p are off by at most 7 u |p|, |v|^2 by 6 u and the distance
+// coordinates of p are off by at most 8 u |p|, |v|^2 by 12 u and the distance
 // and its square by a few u more; the boxes carry the triangles' own rounding
-// (build_frames).  2^-20 |p|_1 = 16 u |p|_1 and a factor 1 + 2^-18 cover these
-// twice over, so no triangle that ties the best distance is pruned.  At most
-// FLT_MAX, which an empty slot's infinite distance exceeds.
+// (build_frames).  2^-20 |p|_1 = 16 u |p|_1 and a factor 1 + 2^-17 cover these
+// twice over, so no triangle that ties the best distance is pruned.
 __device__ __forceinline__ float prune_limit(float best, V3 p) {
   float s;
   asm("sqrt.approx.f32 %0, %1;" : "=f"(s) : "f"(best));
   s = fmaf(fabsf(p.x) + fabsf(p.y) + fabsf(p.z), 9.5367431640625e-07f, s);
-  return fminf(s * s * 1.000003814697265625f, FLT_MAX);
+  return fminf(s * s * 1.00000762939453125f, FLT_MAX);
 }
 
 struct ClosestHit {
@@ -271,12 +363,9 @@ struct ClosestHit {
 // (d2, id) order.  Seeding a query with real candidates gives the traversal a
 // tight bound without changing its answer.  kFast selects the contracted-FP32
 // triangle routine (walker); callers use the test_slot / test_slot_fast wrappers.
-template <bool kFast, bool kL1 = false>
-__device__ __forceinline__ void test_slot_impl(const float4* __restrict__ tris, int slot, V3 p, ClosestHit& hit) {
-  const float4* t = tris + static_cast<size_t>(slot) * 4;
-  float4 r0, r1, r2, r3;
-  ldg_v8f<kL1>(t + 0, r0, r1);
-  ldg_v8f<kL1>(t + 2, r2, r3);
+template <bool kFast>
+__device__ __forceinline__ void test_rec(const Rec64& rec, int slot, V3 p, ClosestHit& hit) {
+  const float4 r0 = rec.r0, r1 = rec.r1, r2 = rec.r2, r3 = rec.r3;
   const V3 a = v3(r0.x, r0.y, r0.z), ab = v3(r1.x, r1.y, r1.z), ac = v3(r1.w, r2.x, r2.y),
            b = v3(r2.z, r2.w, r3.x), c = v3(r3.y, r3.z, r3.w);
   V3 cp;
@@ -300,6 +389,10 @@ __device__ __forceinline__ void test_slot_impl(const float4* __restrict__ tris, 
   }
 }
 
+template <bool kFast, bool kL1 = false>
+__device__ __forceinline__ void test_slot_impl(const float4* __restrict__ tris, int slot, V3 p, ClosestHit& hit) {
+  test_rec<kFast>(load_rec<kL1>(tris, slot), slot, p, hit);
+}
 __device__ __forceinline__ void test_slot(const float4* __restrict__ tris, int slot, V3 p, ClosestHit& hit) {
   test_slot_impl<false>(tris, slot, p, hit);
 }
@@ -556,43 +649,78 @@ __device__ __forceinline__ void trav_triangle(const float4* __restrict__ tris, V
 // Expands one pending node, if there is one and the leaf list has room.  The
 // children within the limit go to the lists by predicated stores (branches per
 // child left 9 of 32 lanes active), the last inner one is entered.
+// Adds the children of a node that are within the limit to the lists.
+__device__ __forceinline__ void expand_node(const Rec64& rec, V3 p, const ClosestHit& hit, FrameTrav& t, FrameStack& st,
+                                            bool& overflow) {
+  const FrameData f = decode_frame_node(rec);
+  float d[4];
+  frame_distances(f, p, d);
+  const int4 ch = f.ch;
+  const bool k0 = d[0] <= hit.lim, k1 = d[1] <= hit.lim, k2 = d[2] <= hit.lim, k3 = d[3] <= hit.lim;
+  const bool n0 = k0 && ch.x >= 0, n1 = k1 && ch.y >= 0, n2 = k2 && ch.z >= 0, n3 = k3 && ch.w >= 0;
+  const bool l0 = k0 && is_leaf(ch.x), l1 = k1 && is_leaf(ch.y), l2 = k2 && is_leaf(ch.z), l3 = k3 && is_leaf(ch.w);
+  if (l0) st.leaves[t.lp] = ch.x;
+  t.lp += l0 ? 1 : 0;
+  if (l1) st.leaves[t.lp] = ch.y;
+  t.lp += l1 ? 1 : 0;
+  if (l2) st.leaves[t.lp] = ch.z;
+  t.lp += l2 ? 1 : 0;
+  if (l3) st.leaves[t.lp] = ch.w;
+  t.lp += l3 ? 1 : 0;
+  const bool p2 = n2 && n3, p1 = n1 && (n2 || n3), p0 = n0 && (n1 || n2 || n3);
+  t.ref = n3 ? ch.w : (n2 ? ch.z : (n1 ? ch.y : (n0 ? ch.x : kEmptyChild)));
+  if (p0) st.nodes[t.np] = ch.x;
+  t.np += p0 ? 1 : 0;
+  if (p1) st.nodes[t.np] = ch.y;
+  t.np += p1 ? 1 : 0;
+  if (p2) st.nodes[t.np] = ch.z;
+  t.np += p2 ? 1 : 0;
+  if (t.np > kTraversalStack) {  // the array holds three more than the limit
+    t.np = kTraversalStack;
+    overflow = true;
+  }
+}
+
 template <bool kL1 = false>
 __device__ __forceinline__ void trav_node(const float4* __restrict__ frames, V3 p, const ClosestHit& hit, FrameTrav& t,
                                           FrameStack& st, uint32_t& c_nodes, bool& overflow) {
   if (t.ref == kEmptyChild && t.np > 0) t.ref = st.nodes[--t.np];
   if (t.ref != kEmptyChild && t.lp <= kLeafRoom) {
-    float4 lox, hix, loy, hiy, loz, hiz;
-    int4 ch;
-    V3 v;
-    load_frame_node<kL1>(frames, t.ref, lox, hix, loy, hiy, loz, hiz, ch, v);
     ++c_nodes;
-    const V3 q = to_frame(v, p);
-    const bool k0 = box_d2_fast(q, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x) <= hit.lim;
-    const bool k1 = box_d2_fast(q, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y) <= hit.lim;
-    const bool k2 = box_d2_fast(q, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z) <= hit.lim;
-    const bool k3 = box_d2_fast(q, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w) <= hit.lim;
-    const bool n0 = k0 && ch.x >= 0, n1 = k1 && ch.y >= 0, n2 = k2 && ch.z >= 0, n3 = k3 && ch.w >= 0;
-    const bool l0 = k0 && ch.x < 0, l1 = k1 && ch.y < 0, l2 = k2 && ch.z < 0, l3 = k3 && ch.w < 0;
-    if (l0) st.leaves[t.lp] = ch.x;
-    t.lp += l0 ? 1 : 0;
-    if (l1) st.leaves[t.lp] = ch.y;
-    t.lp += l1 ? 1 : 0;
-    if (l2) st.leaves[t.lp] = ch.z;
-    t.lp += l2 ? 1 : 0;
-    if (l3) st.leaves[t.lp] = ch.w;
-    t.lp += l3 ? 1 : 0;
-    const bool p2 = n2 && n3, p1 = n1 && (n2 || n3), p0 = n0 && (n1 || n2 || n3);
-    t.ref = n3 ? ch.w : (n2 ? ch.z : (n1 ? ch.y : (n0 ? ch.x : kEmptyChild)));
-    if (p0) st.nodes[t.np] = ch.x;
-    t.np += p0 ? 1 : 0;
-    if (p1) st.nodes[t.np] = ch.y;
-    t.np += p1 ? 1 : 0;
-    if (p2) st.nodes[t.np] = ch.z;
-    t.np += p2 ? 1 : 0;
-    if (t.np > kTraversalStack) {  // the array holds three more than the limit
-      t.np = kTraversalStack;
-      overflow = true;
-    }
+    expand_node(load_rec<kL1>(frames, t.ref), p, hit, t, st, overflow);
+  }
+}
+
+// trav_triangle and trav_node with both records loaded before either is used:
+// one memory latency per step, for launches of so few walks that registers are
+// plentiful and latency is all there is.
+template <bool kFast, bool kL1>
+__device__ __forceinline__ void trav_both(const float4* __restrict__ frames, const float4* __restrict__ tris, V3 p,
+                                          ClosestHit& hit, FrameTrav& t, FrameStack& st, uint32_t& c_nodes,
+                                          uint32_t& c_tris, bool& overflow) {
+  if (t.leaf_cur >= t.leaf_end && t.lp > 0) {
+    const int e = st.leaves[--t.lp];
+    t.leaf_cur = leaf_first(e);
+    t.leaf_end = t.leaf_cur + leaf_count(e);
+  }
+  if (t.ref == kEmptyChild && t.np > 0) t.ref = st.nodes[--t.np];
+  const bool has_node = t.ref != kEmptyChild && t.lp <= kLeafRoom;
+  bool has_tri = t.leaf_cur < t.leaf_end;
+  const int slot = t.leaf_cur;
+  if (has_tri) {
+    ++t.leaf_cur;
+    has_tri = slot != hit.slot;
+  }
+  Rec64 tri, node;
+  if (has_tri) tri = load_rec<kL1>(tris, slot);
+  if (has_node) node = load_rec<kL1>(frames, t.ref);
+  if (has_tri) {
+    test_rec<kFast>(tri, slot, p, hit);
+    ++c_tris;
+  }
+  if (has_node) {
+    ++c_nodes;
+    expand_node(node, p, hit, t, st, overflow);
   }
 }
 

@@ -466,8 +466,12 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
       if (busy == 0 || __popc(waiting) >= a.regen) break;
       if (querying) {
         bool ov = false;
-        dev::trav_triangle<true, kL1>(a.tris, x, hit, tv, stack, c_tris);
-        dev::trav_node<kL1>(a.nodes, x, hit, tv, stack, c_nodes, ov);
+        if constexpr (kL1) {
+          dev::trav_both<true, kL1>(a.nodes, a.tris, x, hit, tv, stack, c_nodes, c_tris, ov);
+        } else {
+          dev::trav_triangle<true>(a.tris, x, hit, tv, stack, c_tris);
+          dev::trav_node(a.nodes, x, hit, tv, stack, c_nodes, ov);
+        }
         querying = !tv.done();
         if (ov) {
           w_overflow = true;
@@ -652,7 +656,10 @@ namespace {
 // 10 / 300 / 1,000 / 2,000 points x 16 walks 1,310 / 2,237 / 2,239 / 2,405 -> 736 /
 // 1,653 / 1,829 / 2,129 us; 4 / 8 / 32 / 64 warps per SM: 728 / 696 / 692 / 691 us
 // and 2,408 / 2,173 / 2,238 / 2,447 us for the first and the last.
+// They load a step's node and triangle together (128 registers; 300 / 1,000 points
+// x 16 walks 1,971 / 2,160 -> 1,591 / 1,707 us).
 constexpr int kSpreadWarps = 16;
+constexpr int kSpreadMinBlocks = 2;
 
 template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks, bool kL1 = false>
 void launch_walker_kernel(WalkArgs a, int block, int blocks_per_sm, cudaStream_t stream) {
@@ -679,7 +686,7 @@ void launch_walker(WalkArgs a, int block, int blocks_per_sm, cudaStream_t stream
     if (lanes < 32) {
       a.lanes = static_cast<int>(lanes);
       a.regen = std::max(1, a.regen * a.lanes / 32);
-      return launch_walker_kernel<kOut, kWalk, kBatch, kMinBlocks, true>(a, block, blocks_per_sm, stream);
+      return launch_walker_kernel<kOut, kWalk, kBatch, kSpreadMinBlocks, true>(a, block, blocks_per_sm, stream);
     }
   }
   launch_walker_kernel<kOut, kWalk, kBatch, kMinBlocks>(a, block, blocks_per_sm, stream);

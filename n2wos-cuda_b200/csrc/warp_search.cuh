@@ -69,15 +69,10 @@ __device__ __forceinline__ void warp_search(const float4* __restrict__ frames, c
     if (e.x != kEmptyChild && __int_as_float(e.y) <= bound) {
       if (e.x >= 0) {
         ++b.nodes;
-        float4 lox, hix, loy, hiy, loz, hiz;
-        int4 ch;
-        V3 v;
-        load_frame_node(frames, e.x, lox, hix, loy, hiy, loz, hiz, ch, v);
-        const V3 f = to_frame(v, p);
-        const float d[4] = {box_d2_fast(f, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x),
-                            box_d2_fast(f, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y),
-                            box_d2_fast(f, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z),
-                            box_d2_fast(f, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w)};
+        const FrameData f = load_frame_node(frames, e.x);
+        float d[4];
+        frame_distances(f, p, d);
+        const int4 ch = f.ch;
         const int r[4] = {ch.x, ch.y, ch.z, ch.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
