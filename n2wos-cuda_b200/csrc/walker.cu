@@ -117,6 +117,70 @@ __device__ __forceinline__ float ball_source(const n2w_problem& pb, uint32_t k0,
   return (R * R) * (1.0f / 6.0f) * f;
 }
 
+// ball_source for a whole warp: the samples of the moving lanes' balls are dealt
+// out over all 32 lanes.  With several samples per ball they are most of a walk
+// update (~250 instructions each), which otherwise runs at the share of lanes
+// that wait for one.  `want`: this lane's ball is sampled; every wanting lane has
+// the same sample count K.  Task t = k n + j is sample k of the j-th wanting
+// lane, so each owner receives its samples in ascending k and adds them in the
+// order ball_source does.  Returns the lane's contribution.  10,000 points x 128
+// walks with 16 samples: 16.8 -> 15.3 ms.
+template <bool kBatch>
+__device__ __forceinline__ float warp_ball_source(bool want, int K, dev::V3 x, float R, uint64_t wid, int step,
+                                                  uint32_t u2, int inst, const WalkArgs& a) {
+  const unsigned mask = __ballot_sync(0xffffffffu, want);
+  const int lane = threadIdx.x & 31, n = __popc(mask);
+  // lane i holds the lane number of the i-th wanting lane
+  int owner_of = 0;
+#pragma unroll
+  for (int b = 16; b > 0; b >>= 1) {
+    if (__popc(mask & ((1u << (owner_of + b)) - 1u)) <= lane) owner_of += b;
+  }
+  int j = lane % n, k = lane / n;                           // this lane's task
+  int off = __popc(mask & ((1u << lane) - 1u));             // lane of this owner's first task in the round
+  const int dj = 32 % n, dk = 32 / n, rounds = 31 / n + 1;  // tasks of one owner in a round
+  float f = 0.0f;
+  for (int t0 = 0; t0 < n * K; t0 += 32) {
+    const int o = __shfl_sync(0xffffffffu, owner_of, j);
+    const dev::V3 xo = dev::v3(__shfl_sync(0xffffffffu, x.x, o), __shfl_sync(0xffffffffu, x.y, o),
+                               __shfl_sync(0xffffffffu, x.z, o));
+    const float Ro = __shfl_sync(0xffffffffu, R, o);
+    const uint32_t w0 = __shfl_sync(0xffffffffu, static_cast<uint32_t>(wid), o);
+    const uint32_t w1 = __shfl_sync(0xffffffffu, static_cast<uint32_t>(wid >> 32), o);
+    const uint32_t so = __shfl_sync(0xffffffffu, static_cast<uint32_t>(step), o);
+    const uint32_t uo = __shfl_sync(0xffffffffu, u2, o);
+    const int io = kBatch ? __shfl_sync(0xffffffffu, inst, o) : 0;
+    float v = 0.0f;
+    if (k < K) {
+      uint32_t k0 = a.k0, k1 = a.k1;
+      const n2w_problem* pb = &a.problem;
+      if constexpr (kBatch) {
+        k0 = a.insts[io].k0;
+        k1 = a.insts[io].k1;
+        pb = a.insts[io].problem;
+      }
+      const U4 r = philox4x32_10(U4{w0, w1, so, 1u + static_cast<uint32_t>(k)}, k0, k1);
+      const float rho = Ro * green_radius_fraction(u01(k == 0 ? uo : r.x));
+      const dev::V3 w = unit_sphere(k == 0 ? r.x : r.y, k == 0 ? r.y : r.z);
+      v = source_f_sample(*pb, xo.x + rho * w.x, xo.y + rho * w.y, xo.z + rho * w.z);
+    }
+    for (int r = 0, l = off; r < rounds; ++r, l += n) {
+      const float s = __shfl_sync(0xffffffffu, v, l & 31);
+      if (want && l < 32 && t0 + l < n * K) f += s;
+    }
+    j += dj;
+    k += dk;
+    if (j >= n) {
+      j -= n;
+      ++k;
+    }
+    off -= dj;
+    if (off < 0) off += n;
+  }
+  if (K > 1) f *= 1.0f / static_cast<float>(K);
+  return (R * R) * (1.0f / 6.0f) * f;
+}
+
 // Adds to point pid's FP64 totals (pid is the global point index; in batched
 // launches instance `inst` owns the accumulators).
 template <bool kBatch>
@@ -391,7 +455,13 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
     //     included, takes its step in this one pass (a finished lane that looped
     //     for its next walk's step ran the whole pass again, nearly alone).  A walk
     //     that ends at its first query waits for the next Phase A.
-    if (alive && !querying && !at_end()) {
+    const bool moving = alive && !querying && !at_end();
+    float R = 0.0f;
+    dev::V3 dir = dev::v3(0.0f, 0.0f, 0.0f);
+    uint32_t u2 = 0;
+    int samples = 0;  // in-ball source samples of this lane's step
+    bool centre = false;
+    if (moving) {
       ++c_queries;
       if (kWalk == N2W_WALK_RESIDUAL && step == a.depth_m && !has_xm) {
         // X_m reached: remember it and the prefix source; the continuation gets a
@@ -401,7 +471,7 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
         has_xm = true;
         cont0 = step;
       }
-      const float R = a.step_scale * dist;
+      R = a.step_scale * dist;
       uint32_t k0 = a.k0, k1 = a.k1;
       if constexpr (kBatch) {
         k0 = a.insts[inst].k0;
@@ -410,12 +480,40 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
       const U4 r = philox4x32_10(U4{static_cast<uint32_t>(wid), static_cast<uint32_t>(wid >> 32),
                                     static_cast<uint32_t>(step), 0u},
                                  k0, k1);
-      const dev::V3 dir = unit_sphere(r.x, r.y);
+      dir = unit_sphere(r.x, r.y);
+      u2 = r.z;
       if constexpr (kBatch) {
         const BatchInst& I = a.insts[inst];
-        if (I.has_source) src += ball_source(*I.problem, k0, k1, I.source_center, I.source_samples, x, R, wid, step, r.z);
+        centre = I.has_source && I.source_center;
+        samples = I.has_source && !I.source_center ? I.source_samples : 0;
       } else {
-        if (a.has_source) src += ball_source(a.problem, k0, k1, a.source_center, a.source_samples, x, R, wid, step, r.z);
+        centre = a.has_source && a.source_center;
+        samples = a.has_source && !a.source_center ? a.source_samples : 0;
+      }
+    }
+    // Several samples per ball: shared by the warp if its lanes agree on the count.
+    const unsigned sampling = __ballot_sync(0xffffffffu, samples >= kManySamples);
+    bool shared = false;
+    if (sampling) {
+      const int K = __shfl_sync(0xffffffffu, samples, __ffs(sampling) - 1);
+      shared = __all_sync(0xffffffffu, samples < kManySamples || samples == K);
+      if (shared) {
+        const bool mine = samples >= kManySamples;
+        const float s = warp_ball_source<kBatch>(mine, K, x, R, wid, step, u2, inst, a);
+        if (mine) {
+          src += s;
+          samples = 0;
+        }
+      }
+    }
+    if (moving) {
+      if (samples > 0 || centre) {
+        if constexpr (kBatch) {
+          const BatchInst& I = a.insts[inst];
+          src += ball_source(*I.problem, I.k0, I.k1, I.source_center, I.source_samples, x, R, wid, step, u2);
+        } else {
+          src += ball_source(a.problem, a.k0, a.k1, a.source_center, a.source_samples, x, R, wid, step, u2);
+        }
       }
       const int prev_slot = hit.slot;
       const dev::V3 xn = dev::v3(x.x + R * dir.x, x.y + R * dir.y, x.z + R * dir.z);
@@ -778,8 +876,7 @@ WalkArgs make_walk_args(const n2w_bvh& bvh, const n2w_problem& problem, const n2
   a.walks_per_point = o.walks_per_point;
   a.chunk = o.chunk > 0 ? std::min(o.chunk, o.walks_per_point) : std::min(kDefaultChunk, o.walks_per_point);
   a.chunks_per_point = (o.walks_per_point + a.chunk - 1) / a.chunk;
-  const bool many_samples = problem_has_source(problem) && problem.source_samples >= kManySamples;
-  a.regen = o.regen_threshold > 0 ? o.regen_threshold : (many_samples ? kManySamplesRegen : kDefaultRegen);
+  a.regen = o.regen_threshold > 0 ? o.regen_threshold : kDefaultRegen;
   a.total_chunks = point_count * a.chunks_per_point;
   a.max_steps = o.max_steps;
   a.depth_m = o.depth_m;

@@ -29,12 +29,11 @@ constexpr int kDefaultChunk = 1;
 // Waiting lanes that make a warp leave the traversal for the walk update: more
 // lanes share the update, fewer traverse meanwhile.  8 / 12 / 14 / 16 / 20:
 // 47.8 / 46.3 / 46.2 / 46.2 / 47.2 ms (Poisson slice, 5.1 M walks), 39.2 / 37.9 /
-// 37.5 / 37.4 / 37.4 ms (batched instances).  With several source samples per
-// ball the update is the longer part: 16 samples, 8 / 12 / 16 / 20 / 24 / 28:
-// 21.6 / 18.3 / 16.9 / 16.3 / 16.3 / 17.1 ms.
+// 37.5 / 37.4 / 37.4 ms (batched instances); 16 samples per ball, 8 / 12 / 16 / 20:
+// 16.5 / 15.7 / 15.3 / 15.5 ms.
 constexpr int kDefaultRegen = 16;
+// Source samples per ball from which a warp shares them (warp_ball_source).
 constexpr int kManySamples = 4;
-constexpr int kManySamplesRegen = 20;
 
 // One instance of a batched launch: its geometry inside the merged scene, its
 // problem, its points and accumulators, and its slice of the global chunk queue.
