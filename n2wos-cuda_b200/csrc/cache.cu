@@ -656,22 +656,20 @@ __global__ void __launch_bounds__(kTrainBlock) train_kernel(const NetArgs a) {
 // Adam (Kingma & Ba) on FP32 master parameters; refreshes the FP16 copy and
 // clears the gradient.  Four parameters per thread in 128-bit accesses: the
 // parameter count is a multiple of 8 (build_meta).  34 bytes per parameter: 12.2 M
-// parameters 102 -> 79 us with the wide accesses, 59 us (7.0 TB/s, part of it L2
-// hits; 6.4 measured copy) with the form of the step below.
-// The step lr (m / bc1) / (sqrt(v / bc2) + eps) is evaluated as c1 m / (sqrt(v) + c2)
-// with c1 = lr sqrt(bc2) / bc1 (a float and its remainder) and c2 = eps sqrt(bc2)
-// from the host: fewer FP32 roundings (RMS error 4.5e-8 against 5.3e-8 over steps
-// of all sizes), and one division and a root instead of three divisions and a
-// root, which had the kernel issue-bound (81 % busy).
+// parameters 102 -> 79 us, 5.3 TB/s (6.4 measured copy).
 struct AdamArgs {
-  float b1, b2, gscale, c1, c1_rest, c2;
+  float lr, b1, b2, eps, bc1, bc2, gscale;
 };
 
-__device__ __forceinline__ void adam_update(float& p, float g, float& m, float& v, const AdamArgs& a) {
+__device__ __forceinline__ float adam_update(float& p, float g, float& m, float& v, const AdamArgs& a) {
   const float gi = g * a.gscale;
-  m = a.b1 * m + (1.0f - a.b1) * gi;
-  v = a.b2 * v + (1.0f - a.b2) * gi * gi;
-  p -= fmaf(a.c1, m, a.c1_rest * m) / (sqrtf(v) + a.c2);
+  const float mi = a.b1 * m + (1.0f - a.b1) * gi;
+  const float vi = a.b2 * v + (1.0f - a.b2) * gi * gi;
+  m = mi;
+  v = vi;
+  const float upd = a.lr * (mi / a.bc1) / (sqrtf(vi / a.bc2) + a.eps);
+  p = p - upd;
+  return p;
 }
 
 __global__ void __launch_bounds__(256) adam_kernel(float4* __restrict__ p, uint2* __restrict__ ph,
@@ -805,15 +803,12 @@ NetArgs net_args(const n2w_cache& c) {
 void launch_adam(n2w_cache& c, float gscale, cudaStream_t s) {
   ++c.step;
   AdamArgs a{};
+  a.lr = c.cfg.learning_rate;
   a.b1 = c.cfg.beta1;
   a.b2 = c.cfg.beta2;
-  const float bc1 = 1.0f - std::pow(a.b1, static_cast<float>(c.step));
-  const float bc2 = 1.0f - std::pow(a.b2, static_cast<float>(c.step));
-  const double root = std::sqrt(static_cast<double>(bc2));
-  const double c1 = static_cast<double>(c.cfg.learning_rate) * root / static_cast<double>(bc1);
-  a.c1 = static_cast<float>(c1);
-  a.c1_rest = static_cast<float>(c1 - static_cast<double>(a.c1));
-  a.c2 = static_cast<float>(static_cast<double>(c.cfg.epsilon) * root);
+  a.eps = c.cfg.epsilon;
+  a.bc1 = 1.0f - std::pow(a.b1, static_cast<float>(c.step));
+  a.bc2 = 1.0f - std::pow(a.b2, static_cast<float>(c.step));
   a.gscale = gscale;
   const int64_t quads = c.n_total / 4;
   const int b = 256;
