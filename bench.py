@@ -13,8 +13,8 @@ Green's-function source sampling.  MSE is against the FP64 analytic u.
 value      = walk-steps (ball moves) of all ranks / max-over-ranks device time
 e2e        = same metric through the C ABI with host buffers: pinned H2D of the
              points and D2H of the per-point FP64 sums inside the timed region
-roofline   = walker kernel: algorithmic bytes (node fetches x 128 B + triangle
-             tests x 48 B + point I/O) / kernel time, against the measured HBM
+roofline   = walker kernel: algorithmic bytes (node fetches x 64 B + triangle
+             tests x 64 B + point I/O) / kernel time, against the measured HBM
              copy bandwidth (the BVH working set is L2-resident; see traffic)
 cpu_baseline = the oracle's scalar WoS port (same walk, CPU BVH) on the host
              cores, bounded sample of the same workload
@@ -226,8 +226,9 @@ def closest_point_segment(n2w, call, stream, timer, flush, cache_peaks, repeat=2
     128 x 256 (65,024 triangles), normalised; 4-wide SAH BVH, leaves of <= 4.
     Each timed launch of n2w_bvh_query_device follows a 256 MiB L2 flush and is
     timed with CUDA events on its stream.  Algorithmic bytes per query:
-    12 in + 28 out + node visits x 128 + triangle tests x 48 (counts from the
-    counting variant of the same traversal).  Beside it, as a baseline, the
+    12 in + 28 out + one 16-byte seed cell + one 64-byte triangle, what any search
+    from the grid reads; the node visits and triangle tests reported beside it are
+    the counted query's, over the axis-aligned nodes.  Beside it, as a baseline, the
     reference's own closest_point_bvh_kernel (src/cuda/bvh_query.cu:75-160,
     median-split BVH, leaf 8, block 128), compiled from its sources for sm_100a,
     on the same points with the same flush."""
@@ -259,7 +260,7 @@ def closest_point_segment(n2w, call, stream, timer, flush, cache_peaks, repeat=2
     d2 = dd.download(np.float32, n, stream)
     ids = di.download(np.int32, n, stream)
     ref = mesh.closest_point_host(pts[:validate])
-    bytes_q = n * (12 + 28) + visits * 128.0 + tests * 48.0
+    bytes_q = n * (12.0 + 28.0 + 16.0 + 64.0)
     med = float(np.median(ms))
     achieved = bytes_q / (med / 1e3) / 1e9
     hbm, hbm_kind = peaks()
@@ -267,7 +268,8 @@ def closest_point_segment(n2w, call, stream, timer, flush, cache_peaks, repeat=2
                        "r=1+0.08 sin6t cos8p 128x256 normalised (65,024 triangles), 4-wide SAH BVH leaf<=4, "
                        "L2 flushed before every timed launch",
            "queries_per_s": n / (med / 1e3), "kernel_ms_median": med, "kernel_ms_min": float(np.min(ms)),
-           "per_query": {"node_visits": visits / n, "tri_tests": tests / n, "algorithmic_bytes": bytes_q / n},
+           "per_query": {"counted_node_visits": visits / n, "counted_tri_tests": tests / n,
+                         "algorithmic_bytes": bytes_q / n},
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                         "peak_source": hbm_kind, "fractions": fractions(achieved, hbm, cache_peaks),
                         "kernel": "closest_point_kernel"},
@@ -791,7 +793,7 @@ def run_batch(args):
     lib.n2w_free_host(hout)
 
     kernel_ms = float(np.mean(times))
-    alg_bytes = c_last["node_visits"] * 128.0 + c_last["tri_tests"] * 48.0 + total_pts * (12 + 8 + 8 + 4 + 8 + 4)
+    alg_bytes = c_last["node_visits"] * 64.0 + c_last["tri_tests"] * 64.0 + total_pts * (12 + 8 + 8 + 4 + 8 + 4)
     achieved = alg_bytes / (kernel_ms / 1e3) / 1e9
     peak, peak_kind = peaks()
     valid = [m for m in mses if m is not None]
@@ -1209,7 +1211,7 @@ def main():
 
     c_last = counters[-1]
     kernel_ms = float(np.mean(times))
-    alg_bytes = c_last["node_visits"] * 128.0 + c_last["tri_tests"] * 48.0 + n * (12 + 8 + 8 + 4 + 8 + 4)
+    alg_bytes = c_last["node_visits"] * 64.0 + c_last["tri_tests"] * 64.0 + n * (12 + 8 + 8 + 4 + 8 + 4)
     achieved = alg_bytes / (kernel_ms / 1e3) / 1e9
     peak, peak_kind = peaks()
     cache_peaks = cache_level_peaks(call)
