@@ -5,11 +5,12 @@
 // (src/geometry/closest_point.cpp:7-48, device twin src/cuda/bvh_query.cu:33-73).
 // Every arithmetic step uses a round-to-nearest intrinsic (__fadd_rn etc.), which
 // the compiler never fuses into an FMA, so results are bit-identical to the
-// reference's g++ build of the same expressions.  The box distance uses the
-// same non-fused operations, which keeps it a rounding-monotone lower bound of
-// every contained triangle's computed distance: pruning with `box_d2 > best_d2`
-// therefore never drops a triangle whose distance ties the current best, and the
-// (d2, id) tie-break returns the lowest triangle id among exact ties — the
+// reference's g++ build of the same expressions.  The axis-aligned box distance
+// uses the same non-fused operations, which keeps it a rounding-monotone lower
+// bound of every contained triangle's computed distance; over the frame nodes
+// prune_limit adds a margin for the frame's rounding.  Pruning therefore never
+// drops a triangle whose distance ties the current best, and the (d2, id)
+// tie-break returns the lowest triangle id among exact ties — the
 // answer of the reference brute force, which keeps the first minimum in index
 // order (closest_point.cpp:57-65).
 #pragma once

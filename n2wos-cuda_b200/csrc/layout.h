@@ -2,8 +2,7 @@
 //
 // Node (128 B, one L2 line): six float4 rows hold the four child boxes in
 // structure-of-arrays form (lo.x, hi.x, lo.y, hi.y, lo.z, hi.z), one int4 row
-// holds the child references, the last 16 B are padding.  A thread fetches the
-// 112 used bytes with seven 16-byte vector loads.
+// holds the child references, the last 16 B are padding.
 //
 // Child reference r:  r >= 0      inner node index
 //                     r == kEmpty  unused slot (its box is +inf/-inf)

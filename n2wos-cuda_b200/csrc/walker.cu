@@ -16,10 +16,10 @@
 //  * the first query of every walk of a point is computed once per point
 //    (exact arithmetic); every later query is seeded with two real candidate
 //    triangles (the previous closest one and the seed-grid one at x), which
-//    bounds the traversal to the walker's neighbourhood, and runs the
-//    contracted-FP32 box and triangle routines of geom.cuh (FMA, fast
-//    division; within a few ulps of the exact query, as the reference's own
-//    nvcc-compiled walker is);
+//    bounds the traversal to the walker's neighbourhood, starts at the subtrees
+//    of x's seed cell, and runs the contracted-FP32 triangle routine of geom.cuh
+//    (FMA, fast division; within a few ulps of the exact query, as the
+//    reference's own nvcc-compiled walker is) over the frame nodes;
 //  * per-point FP64 sum / sum of squares accumulated per lane over its chunk,
 //    merged across lanes with warp shuffles and flushed with FP64 atomics.
 #include <cuda_runtime.h>
