@@ -163,14 +163,6 @@ __device__ __forceinline__ V3 closest_point_triangle_fast(V3 p, V3 a, V3 b, V3 c
   return r;
 }
 
-__device__ __forceinline__ float box_d2_fast(V3 p, float lox, float hix, float loy, float hiy, float loz,
-                                             float hiz) {
-  const float dx = p.x - fminf(fmaxf(p.x, lox), hix);
-  const float dy = p.y - fminf(fmaxf(p.y, loy), hiy);
-  const float dz = p.z - fminf(fmaxf(p.z, loz), hiz);
-  return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-}
-
 __device__ __forceinline__ void cswap(float& da, int& ra, float& db, int& rb) {
   if (db < da) {
     const float td = da;
