@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kerne
       overflow = false;
       int4 cell = make_int4(0, 0, kEmptyChild, kEmptyChild);  // the root
       if (grid.cells) {
-        cell = dev::seed_cell(grid, p, 0);
+        cell = kCount ? dev::seed_cell(grid, p, 0) : dev::seed_cell_any(grid, p, 0);
         dev::test_slot(tris, cell.x, p, hit);
         ++c_tris;
       }
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) closest_point_finish
     b.cp = dev::v3(c0.x, c0.y, c0.z);
     b.slot = -1;
     int4 start = make_int4(0, 0, kEmptyChild, kEmptyChild);  // the root
-    if (grid.cells) start = dev::seed_cell(grid, p, 0);
+    if (grid.cells) start = dev::seed_cell_any(grid, p, 0);
     dev::warp_search(nodes, tris, p, start, b, work);
     if (b.winner()) {
       const int id = static_cast<int>(b.key & 0xffffffffu);

@@ -409,7 +409,8 @@ struct SeedGrid {
 };
 
 // The cell of the lattice node nearest to p; outside the lattice the clamped
-// node's cell with the root as its only subtree.
+// node's cell with the root as its only subtree.  (Walks stay inside; the counted
+// query's seeds, which the CPU restatement reproduces.)
 __device__ __forceinline__ int4 seed_cell(const SeedGrid& g, V3 p, int root) {
   const float fx = (p.x - g.lo_x) * g.inv_h, fy = (p.y - g.lo_y) * g.inv_h, fz = (p.z - g.lo_z) * g.inv_h;
   const float n = static_cast<float>(g.n);
@@ -417,6 +418,30 @@ __device__ __forceinline__ int4 seed_cell(const SeedGrid& g, V3 p, int root) {
   const int s = g.n + 1;
   int4 c = __ldg(g.cells + (static_cast<size_t>(__float2int_rn(cz)) * s + __float2int_rn(cy)) * s + __float2int_rn(cx));
   if (!(cx == fx && cy == fy && cz == fz)) {
+    c.y = root;
+    c.z = c.w = kEmptyChild;
+  }
+  return c;
+}
+
+// The same for any point: outside the lattice the cell where the ray from the
+// lattice's centre to p leaves it, with the root as its only subtree.  (A point
+// clamped axis by axis lies in another direction from the mesh, and its triangle is
+// a poor seed.)  300,000 queries around 81,920 triangles, 5 extents from their centre:
+// 3,535 -> 869 us, 1.5 extents: 2,017 -> 645 us.
+__device__ __forceinline__ int4 seed_cell_any(const SeedGrid& g, V3 p, int root) {
+  const float half = 0.5f * static_cast<float>(g.n), n = static_cast<float>(g.n);
+  const float fx = (p.x - g.lo_x) * g.inv_h - half, fy = (p.y - g.lo_y) * g.inv_h - half,
+              fz = (p.z - g.lo_z) * g.inv_h - half;
+  const float far = fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz)));
+  const bool in = fabsf(fx) <= half && fabsf(fy) <= half && fabsf(fz) <= half;
+  const float s = in ? 1.0f : half / far;
+  // (not a number: node 0)
+  const float cx = fminf(fmaxf(fmaf(fx, s, half), 0.0f), n), cy = fminf(fmaxf(fmaf(fy, s, half), 0.0f), n),
+              cz = fminf(fmaxf(fmaf(fz, s, half), 0.0f), n);
+  const int m = g.n + 1;
+  int4 c = __ldg(g.cells + (static_cast<size_t>(__float2int_rn(cz)) * m + __float2int_rn(cy)) * m + __float2int_rn(cx));
+  if (!in) {
     c.y = root;
     c.z = c.w = kEmptyChild;
   }
@@ -725,7 +750,7 @@ __device__ __forceinline__ void traverse_frames(const float4* __restrict__ frame
   FrameStack stack;
   FrameTrav t;
   if (grid.cells) {
-    const int4 cell = seed_cell(grid, p, root);
+    const int4 cell = seed_cell_any(grid, p, root);
     test_slot(tris, cell.x, p, hit);
     ++st.tri_tests;
     t.start(cell, stack);

@@ -137,7 +137,7 @@ __device__ __forceinline__ WarpBest warp_query(const float4* __restrict__ frames
   h.cp = no_hit;
   int4 cell = make_int4(0, root, kEmptyChild, kEmptyChild);
   if (grid.cells) {
-    cell = seed_cell(grid, p, root);
+    cell = seed_cell_any(grid, p, root);
     test_slot(tris, cell.x, p, h);
   }
   WarpBest b;

@@ -1,0 +1,54 @@
+"""Closest-point searches from points outside the seed grid's lattice (the mesh box
+grown by 20 %): the answers of the counted query, for a bounded share of its work.
+
+The counted query searches axis-aligned boxes; a plain estimate whose epsilon is
+larger than any distance runs nothing but the points' first queries, and its run
+counters are their node expansions and triangle tests."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SWITCH = 32768  # launches above this many points search with one lane per point
+
+
+def sphere_points(v, n, extents, seed):
+    """Points on the sphere around the mesh's box centre, `extents` times its largest extent away."""
+    rng = np.random.default_rng(seed)
+    lo, hi = v.min(0).astype(float), v.max(0).astype(float)
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1)[:, None]
+    return ((lo + hi) / 2 + d * (hi - lo).max() * extents).astype(np.float32)
+
+
+def first_query_work(gpu, bvh, pts):
+    """(nodes + triangles of the first queries) per point."""
+    o = gpu.walk_options(walks_per_point=1, max_steps=1, epsilon=1e30)
+    _, c = gpu.wos_estimate(bvh, gpu.problem_charges_seeded(8, 1.6, 2.0, 1), pts, options=o)
+    assert c["steps"] == 0 and c["overflow"] == 0
+    return (c["node_visits"] + c["tri_tests"]) / len(pts)
+
+
+def assert_same_answers(got, want):
+    for k in ("distance2", "closest"):
+        assert np.array_equal(got[k].view(np.uint32), want[k].view(np.uint32)), k
+    assert np.array_equal(got["triangle_id"], want["triangle_id"])
+    assert not got["overflow"].any()
+
+
+@pytest.fixture(scope="module")
+def sphere(gpu):
+    m = gpu.Mesh.icosphere_displaced(5, 0.12, 3.0, 4, 0.5, 12345)
+    return gpu.Bvh(m, 4, "sah"), m.arrays()[0]
+
+
+@pytest.mark.parametrize("extents", [1.5, 5.0])
+def test_seeds_outside_the_lattice(gpu, sphere, extents):
+    """The seed lies in the direction of the point, so the search does half of the counted query's work or less."""
+    bvh, v = sphere
+    pts = sphere_points(v, SWITCH + 37, extents, 3)
+    want = bvh.query(pts, counted=True)
+    assert_same_answers(bvh.query(pts), want)
+    assert_same_answers(bvh.query(pts[:1000]), {k: x[:1000] for k, x in want.items()})
+    counted = (want["node_visits"] + want["tri_tests"]).mean()
+    assert first_query_work(gpu, bvh, pts) < 0.5 * counted
