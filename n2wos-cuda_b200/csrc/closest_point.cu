@@ -77,8 +77,8 @@ struct Search {
     // triangles (one node: 372 against 357 us for 262,144 queries, equal for
     // 1,000,003 near the surface and 4,194,304).
     dev::trav_triangle<false>(tris, p, hit, t, stack, c_tris);
-    dev::trav_node(frames, p, hit, t, stack, c_nodes, overflow);
-    dev::trav_node(frames, p, hit, t, stack, c_nodes, overflow);
+    dev::trav_node<false, true>(frames, p, hit, t, stack, c_nodes, overflow);
+    dev::trav_node<false, true>(frames, p, hit, t, stack, c_nodes, overflow);
     return !t.done();
   }
 };

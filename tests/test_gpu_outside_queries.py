@@ -52,3 +52,35 @@ def test_seeds_outside_the_lattice(gpu, sphere, extents):
     assert_same_answers(bvh.query(pts[:1000]), {k: x[:1000] for k, x in want.items()})
     counted = (want["node_visits"] + want["tri_tests"]).mean()
     assert first_query_work(gpu, bvh, pts) < 0.5 * counted
+
+
+def _patch(n, corner, eu, ev):
+    """An n x n grid of quads, two triangles each."""
+    g = np.linspace(0.0, 1.0, n + 1)
+    u, w = (x.reshape(-1, 1) for x in np.meshgrid(g, g, indexing="ij"))
+    v = np.asarray(corner, float) + u * np.asarray(eu, float) + w * np.asarray(ev, float)
+    i = (np.arange(n)[:, None] * (n + 1) + np.arange(n)).ravel()
+    return v, np.concatenate([np.stack([i, i + n + 1, i + 1], -1), np.stack([i + 1, i + n + 1, i + n + 2], -1)])
+
+
+def _join(parts):
+    off = np.cumsum([0] + [len(v) for v, _ in parts])
+    return np.concatenate([v for v, _ in parts]).astype(np.float32), np.concatenate([t + o for (_, t), o in zip(parts, off)])
+
+
+@pytest.fixture(scope="module")
+def cube(gpu):
+    """An axis-aligned cube, sides of 60 x 60 quads."""
+    n, e = 60, 2 * np.eye(3)
+    v, t = _join([_patch(n, -np.ones(3) + side * e[a], e[(a + 1) % 3], e[(a + 2) % 3]) for a in range(3) for side in (0, 1)])
+    return gpu.Bvh(gpu.Mesh.from_arrays(v, t), 4, "sah"), v
+
+
+def test_nearest_children_first(gpu, cube):
+    """Flat sides seen from outside: many triangles lie within the seed's distance, few within the answer's."""
+    bvh, v = cube
+    pts = sphere_points(v, SWITCH + 37, 1.5, 4)
+    want = bvh.query(pts, counted=True)
+    assert_same_answers(bvh.query(pts), want)
+    counted = (want["node_visits"] + want["tri_tests"]).mean()
+    assert first_query_work(gpu, bvh, pts) < 4.0 * counted
