@@ -207,14 +207,29 @@ __device__ __forceinline__ int4 ldg_v8_first_int4(const float4* p) {
       : "l"(p));
   return a;
 }
+template <bool kL1>
 __device__ __forceinline__ void load_node(const float4* __restrict__ nodes, int32_t ref, float4& lox, float4& hix,
                                           float4& loy, float4& hiy, float4& loz, float4& hiz, int4& ch) {
   static_assert(sizeof(Node4) == 128, "node loads assume 128-byte nodes");
   const float4* n = nodes + static_cast<size_t>(ref) * 8;
-  ldg_v8f(n + 0, lox, hix);
-  ldg_v8f(n + 2, loy, hiy);
-  ldg_v8f(n + 4, loz, hiz);
+  ldg_v8f<kL1>(n + 0, lox, hix);
+  ldg_v8f<kL1>(n + 2, loy, hiy);
+  ldg_v8f<kL1>(n + 4, loz, hiz);
   ch = ldg_v8_first_int4(n + 6);
+}
+
+// Squared distances from p to the four child boxes of an axis-aligned node; returns
+// its child references.
+template <bool kL1 = false>
+__device__ __forceinline__ int4 box_distances(const float4* __restrict__ nodes, int32_t ref, V3 p, float (&d)[4]) {
+  float4 lox, hix, loy, hiy, loz, hiz;
+  int4 ch;
+  load_node<kL1>(nodes, ref, lox, hix, loy, hiy, loz, hiz, ch);
+  d[0] = box_d2(p, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x);
+  d[1] = box_d2(p, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y);
+  d[2] = box_d2(p, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z);
+  d[3] = box_d2(p, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w);
+  return ch;
 }
 
 struct Rec64 {  // a 64-byte record as loaded
@@ -448,6 +463,14 @@ __device__ __forceinline__ int4 seed_cell_any(const SeedGrid& g, V3 p, int root)
   return c;
 }
 
+// A tree as queries search it.  The arrays share node indices and leaves, and the
+// answer is the same over either.
+struct QueryNodes {
+  const float4* frames;  // FrameNode4
+  const float4* boxes;   // Node4
+  bool use_boxes;        // the tree's choice (choose_nodes)
+};
+
 struct TraversalStats {
   int node_visits;
   int tri_tests;
@@ -468,6 +491,7 @@ __device__ __forceinline__ void traverse(const float4* __restrict__ nodes,
   int32_t ref = root;
   for (;;) {
     if (ref >= 0) {
+      ++st.node_visits;
       const float4* n = nodes + static_cast<size_t>(ref) * 8;
       const float4 lox = __ldg(n + 0);
       const float4 hix = __ldg(n + 1);
@@ -503,6 +527,7 @@ __device__ __forceinline__ void traverse(const float4* __restrict__ nodes,
     } else if (ref != kEmptyChild) {
       const int first = leaf_first(ref);
       const int count = leaf_count(ref);
+      st.tri_tests += count;
       for (int i = 0; i < count; ++i) test_slot_impl<false>(tris, first + i, p, hit);
       ref = kEmptyChild;
     }
@@ -522,7 +547,8 @@ __device__ __forceinline__ void traverse(const float4* __restrict__ nodes,
 }
 
 // ---- one lane's query over the axis-aligned nodes, unit by unit ----------------
-// (the counted query, whose visit counts the CPU restatement reproduces)
+// (the counted query, whose visit counts the CPU restatement reproduces, and the
+// trees whose frames do not pay)
 struct TravState {
   int sp;
   int ref;       // inner node to expand next, or kEmptyChild
@@ -534,6 +560,7 @@ struct TravState {
 // ONE 4-wide node (same ordering and pruning as dev::traverse: children sorted
 // by box distance, nearest entered, others pushed far-to-near, popped entries
 // re-checked).  Returns false once the query is complete.
+template <bool kL1>
 __device__ __forceinline__ bool trav_step_boxes(const float4* __restrict__ nodes, const float4* __restrict__ tris,
                                                 V3 p, ClosestHit& hit, TravState& t, int2* stack, uint32_t& c_nodes,
                                                 uint32_t& c_tris, bool& overflow) {
@@ -555,19 +582,15 @@ __device__ __forceinline__ bool trav_step_boxes(const float4* __restrict__ nodes
     if (!found) return false;
   }
   if (t.leaf_cur < t.leaf_end) {
-    test_slot_impl<false>(tris, t.leaf_cur, p, hit);
+    test_slot_impl<false, kL1>(tris, t.leaf_cur, p, hit);
     ++t.leaf_cur;
     ++c_tris;
     return true;
   }
-  float4 lox, hix, loy, hiy, loz, hiz;
-  int4 ch;
-  load_node(nodes, t.ref, lox, hix, loy, hiy, loz, hiz, ch);
+  float d[4];
+  const int4 ch = box_distances<kL1>(nodes, t.ref, p, d);
   ++c_nodes;
-  float d0 = box_d2(p, lox.x, hix.x, loy.x, hiy.x, loz.x, hiz.x);
-  float d1 = box_d2(p, lox.y, hix.y, loy.y, hiy.y, loz.y, hiz.y);
-  float d2 = box_d2(p, lox.z, hix.z, loy.z, hiy.z, loz.z, hiz.z);
-  float d3 = box_d2(p, lox.w, hix.w, loy.w, hiy.w, loz.w, hiz.w);
+  float d0 = d[0], d1 = d[1], d2 = d[2], d3 = d[3];
   int r0 = ch.x, r1 = ch.y, r2 = ch.z, r3 = ch.w;
   cswap(d0, r0, d1, r1);
   cswap(d2, r2, d3, r3);
@@ -753,17 +776,21 @@ __device__ __forceinline__ void trav_both(const float4* __restrict__ frames, con
   }
 }
 
-// A whole cold query in one lane over the frame nodes (exact routines), seeded
-// by the grid if there is one.
-__device__ __forceinline__ void traverse_frames(const float4* __restrict__ frames, const float4* __restrict__ tris,
-                                                const SeedGrid& grid, V3 p, ClosestHit& hit, TraversalStats& st,
-                                                int32_t root) {
+// A whole query in one lane (exact routines), seeded by the grid if there is one.
+__device__ __forceinline__ void traverse_query(const QueryNodes& nodes, const float4* __restrict__ tris,
+                                               const SeedGrid& grid, V3 p, ClosestHit& hit, TraversalStats& st,
+                                               int32_t root) {
+  const float4* __restrict__ frames = nodes.frames;
   FrameStack stack;
   FrameTrav t;
   if (grid.cells) {
     const int4 cell = seed_cell_any(grid, p, root);
     test_slot(tris, cell.x, p, hit);
     ++st.tri_tests;
+    if (nodes.use_boxes) {
+      traverse(nodes.boxes, tris, p, hit, st, root);
+      return;
+    }
     t.start(cell, stack);
   } else {
     t.start(root);

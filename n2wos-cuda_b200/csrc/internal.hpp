@@ -20,13 +20,14 @@ struct n2w_mesh {
 
 struct n2w_bvh {
   n2w::Node4* d_nodes = nullptr;         // axis-aligned boxes: ray parity, counted queries, the copied-out layout
-  n2w::FrameNode4* d_frames = nullptr;  // the same tree with boxes in per-node frames: closest-point traversals
+  n2w::FrameNode4* d_frames = nullptr;  // the same tree with boxes in per-node frames: walks, most trees' queries
   n2w::TriRec* d_tris = nullptr;        // leaf-ordered triangles: ray parity, the copied-out layout
   n2w::TriEdges* d_edges = nullptr;     // the same triangles for the closest-point test
   int4* d_seed = nullptr;  // seed grid: nearest triangle's leaf slot and start subtrees per lattice node (geom.cuh)
   float seed_lo[3] = {0, 0, 0};
   float seed_h = 0.0f;
   int seed_n = 0;
+  bool use_boxes = false;  // queries search d_nodes, not d_frames (choose_nodes)
   n2w_bvh_stats stats{};
   int device = 0;
 };

@@ -45,8 +45,9 @@ struct WarpBest {
 
 // Searches the subtrees start.y, start.z, start.w (kEmptyChild when unused) for
 // a hit better than b, which holds the seed in every lane.
-__device__ __forceinline__ void warp_search(const float4* __restrict__ frames, const float4* __restrict__ tris, V3 p,
-                                            int4 start, WarpBest& b, int2* work) {
+template <bool kBoxes>
+__device__ __forceinline__ void warp_search_over(const float4* __restrict__ nodes, const float4* __restrict__ tris,
+                                                 V3 p, int4 start, WarpBest& b, int2* work) {
   const int lane = threadIdx.x & 31;
   b.dropped = 0;
   b.nodes = b.tris = 0;
@@ -63,16 +64,21 @@ __device__ __forceinline__ void warp_search(const float4* __restrict__ frames, c
     if (lane < take) e = work[sp - take + lane];
     __syncwarp();
     sp -= take;
-    const float bound = prune_limit(key_d2(b.key), p);
+    const float bound = kBoxes ? key_d2(b.key) : prune_limit(key_d2(b.key), p);
     int2 c[4];
     int nc = 0;
     if (e.x != kEmptyChild && __int_as_float(e.y) <= bound) {
       if (e.x >= 0) {
         ++b.nodes;
-        const FrameData f = load_frame_node(frames, e.x);
         float d[4];
-        frame_distances(f, p, d);
-        const int4 ch = f.ch;
+        int4 ch;
+        if constexpr (kBoxes) {
+          ch = box_distances(nodes, e.x, p, d);
+        } else {
+          const FrameData f = load_frame_node(nodes, e.x);
+          frame_distances(f, p, d);
+          ch = f.ch;
+        }
         const int r[4] = {ch.x, ch.y, ch.z, ch.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -127,8 +133,14 @@ __device__ __forceinline__ void warp_search(const float4* __restrict__ frames, c
   }
 }
 
+__device__ __forceinline__ void warp_search(const QueryNodes& nodes, const float4* __restrict__ tris, V3 p, int4 start,
+                                            WarpBest& b, int2* work) {
+  if (nodes.use_boxes) warp_search_over<true>(nodes.boxes, tris, p, start, b, work);
+  else warp_search_over<false>(nodes.frames, tris, p, start, b, work);
+}
+
 // A cold query, seeded and started by the grid if there is one.
-__device__ __forceinline__ WarpBest warp_query(const float4* __restrict__ frames, const float4* __restrict__ tris,
+__device__ __forceinline__ WarpBest warp_query(const QueryNodes& nodes, const float4* __restrict__ tris,
                                                const SeedGrid& grid, V3 p, int root, V3 no_hit, int2* work) {
   ClosestHit h;
   h.d2 = h.lim = FLT_MAX;
@@ -144,7 +156,7 @@ __device__ __forceinline__ WarpBest warp_query(const float4* __restrict__ frames
   b.key = b.mine = hit_key(h.d2, h.id);
   b.cp = h.cp;
   b.slot = h.slot;
-  warp_search(frames, tris, p, cell, b, work);
+  warp_search(nodes, tris, p, cell, b, work);
   if (grid.cells && (threadIdx.x & 31) == 0) ++b.tris;
   return b;
 }

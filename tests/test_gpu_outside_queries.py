@@ -84,3 +84,30 @@ def test_nearest_children_first(gpu, cube):
     assert_same_answers(bvh.query(pts), want)
     counted = (want["node_visits"] + want["tri_tests"]).mean()
     assert first_query_work(gpu, bvh, pts) < 4.0 * counted
+
+
+@pytest.fixture(scope="module")
+def needles(gpu):
+    """The side of a cylinder in 2 x 5,000 triangles, each 2 long and 0.001 wide."""
+    k = 5000
+    a = np.arange(k) * 2 * np.pi / k
+    lo = np.stack([np.cos(a), np.sin(a), -np.ones(k)], -1)
+    i, j = np.arange(k), (np.arange(k) + 1) % k
+    t = np.concatenate([np.stack([i, j, i + k], -1), np.stack([j, j + k, i + k], -1)])
+    v = np.concatenate([lo, lo + [0, 0, 2]]).astype(np.float32)
+    return gpu.Bvh(gpu.Mesh.from_arrays(v, t), 4, "sah"), v
+
+
+@pytest.mark.parametrize("n", [1000, SWITCH + 37])
+@pytest.mark.parametrize("where", ["inside", "outside"])
+@pytest.mark.parametrize("name", ["cube", "needles"])
+def test_trees_whose_frames_do_not_pay(gpu, request, name, where, n):
+    """Axis-aligned sides and bundles of needles: the queries search the axis-aligned boxes, from seeds at least as
+    good as the counted query's, so a lane does no more work than that."""
+    bvh, v = request.getfixturevalue(name)
+    pts = np.random.default_rng(6).uniform(-1.2, 1.2, (n, 3)).astype(np.float32) if where == "inside" else \
+        sphere_points(v, n, 1.5, 6)
+    want = bvh.query(pts, counted=True)
+    assert_same_answers(bvh.query(pts), want)
+    if n > SWITCH:
+        assert first_query_work(gpu, bvh, pts) <= 1.0 * (want["node_visits"] + want["tri_tests"]).mean()
