@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <cstring>
 
 #include "geom.cuh"
@@ -26,6 +27,7 @@ dev::SeedGrid seed_grid_of(const n2w_bvh& b) {
   g.lo_z = b.seed_lo[2];
   g.inv_h = b.seed_h > 0.0f ? 1.0f / b.seed_h : 0.0f;
   g.n = b.seed_n;
+  g.far = b.seed_far;
   return g;
 }
 
@@ -61,6 +63,7 @@ constexpr int kQueryBlock = 256;
 constexpr uint32_t kQueryBudget = 112;
 constexpr uint32_t kBoxBudget = 384;  // the same over the boxes, whose long queries have more nodes to visit
 constexpr int kHandOff = 2;         // overflow-slot mark of a handed-off query
+constexpr int kHandOffFar = 3;      // the same for a far one (far_limit), handed off as soon as it is seeded
 // Launches of at most this many queries give each query a warp: with a lane per
 // query a launch lasts as long as its slowest serial search, whatever its size.
 // Lane / warp per query, uniform points, 81,920 triangles: 71 / 11 us (40
@@ -130,6 +133,14 @@ __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kerne
   uint32_t c_nodes = 0, c_tris = 0;
   bool overflow = false;
   Search<kMode> search;
+  // Hands the query to the finisher with its best so far (a bound on the answer) in
+  // its own output slots.
+  auto hand_off = [&](int mark) {
+    out_d2[q] = hit.d2;
+    out_cp[q] = n2w_vec3{hit.cp.x, hit.cp.y, hit.cp.z};
+    out_id[q] = hit.id == INT32_MAX ? -1 : hit.id;
+    out_overflow[q] = mark;
+  };
   for (;;) {
     while (!busy && !drained) {
       const unsigned claim = atomicAdd(&s_next, 1u);
@@ -159,9 +170,14 @@ __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kerne
       overflow = false;
       int4 cell = make_int4(0, 0, kEmptyChild, kEmptyChild);  // the root
       if (grid.cells) {
-        cell = kCount ? dev::seed_cell(grid, p, 0) : dev::seed_cell_any(grid, p, 0);
+        bool far = false;
+        cell = kCount ? dev::seed_cell(grid, p, 0) : dev::seed_cell_any(grid, p, 0, far);
         dev::test_slot(tris, cell.x, p, hit);
         ++c_tris;
+        if (kMode == kFrames && far) {
+          hand_off(kHandOffFar);
+          continue;
+        }
       }
       search.start(cell);
       busy = true;
@@ -169,12 +185,7 @@ __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kerne
     if (!__any_sync(0xffffffffu, busy)) break;
     if (busy) {
       if (!kCount && budget && c_nodes + c_tris > budget) {
-        // Over budget: hand the query to the warp-cooperative finisher with its
-        // best so far (a bound on the answer) in its own output slots.
-        out_d2[q] = hit.d2;
-        out_cp[q] = n2w_vec3{hit.cp.x, hit.cp.y, hit.cp.z};
-        out_id[q] = hit.id == INT32_MAX ? -1 : hit.id;
-        out_overflow[q] = kHandOff;
+        hand_off(kHandOff);  // over budget
         busy = false;
       } else if (!search.step(nodes, tris, p, hit, c_nodes, c_tris, overflow)) {
         out_d2[q] = hit.d2;
@@ -191,11 +202,13 @@ __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kerne
   }
 }
 
-// Finisher for the queries that ran over the per-lane budget (marked kHandOff in
+// Finisher for the queries that ran over the per-lane budget or are far away (marked in
 // their overflow slot): one warp per group of 32 consecutive queries takes its
 // marked queries one at a time and searches again (warp_search.cuh) with the
 // lane's best so far as the bound.  Blocks whose groups hold no marked query
-// exit at once, so the block scheduler balances the work.
+// exit at once, so the block scheduler balances the work.  (A lane per far query
+// instead: 81,920 triangles, 100,003 queries 500 extents away 727 -> 1,335 us, two close
+// sheets of 45,000 triangles 4 -> 50 ms.)
 __global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) closest_point_finish_kernel(
     const dev::QueryNodes nodes, const float4* __restrict__ tris, const dev::SeedGrid grid,
     const n2w_vec3* __restrict__ points, int n, float* __restrict__ out_d2, n2w_vec3* __restrict__ out_cp,
@@ -207,9 +220,11 @@ __global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) closest_point_finish
   const int64_t q0 = (static_cast<int64_t>(blockIdx.x) * dev::kWarpsPerBlock + warp) * 32;
   if (q0 >= n) return;
   const int64_t mine = q0 + lane;
-  unsigned pending = __ballot_sync(0xffffffffu, mine < n && out_overflow[mine] == kHandOff);
+  const int mark = mine < n ? out_overflow[mine] : 0;
+  unsigned pending = __ballot_sync(0xffffffffu, mark >= kHandOff);
+  const unsigned far = __ballot_sync(0xffffffffu, mark == kHandOffFar);
   while (pending) {
-    const int q = static_cast<int>(q0) + __ffs(pending) - 1;
+    const int i = __ffs(pending) - 1, q = static_cast<int>(q0) + i;
     pending &= pending - 1;
     const n2w_vec3 pt = points[q], c0 = out_cp[q];
     const dev::V3 p = dev::v3(pt.x, pt.y, pt.z);
@@ -219,8 +234,9 @@ __global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) closest_point_finish
     b.cp = dev::v3(c0.x, c0.y, c0.z);
     b.slot = -1;
     int4 start = make_int4(0, 0, kEmptyChild, kEmptyChild);  // the root
-    if (grid.cells) start = dev::seed_cell_any(grid, p, 0);
-    dev::warp_search(nodes, tris, p, start, b, work);
+    bool at_far;
+    if (grid.cells) start = dev::seed_cell_any(grid, p, 0, at_far);
+    dev::warp_search(nodes, tris, p, start, (far >> i) & 1u, b, work);
     if (b.winner()) {
       const int id = static_cast<int>(b.key & 0xffffffffu);
       out_d2[q] = dev::key_d2(b.key);
@@ -305,7 +321,7 @@ __global__ void __launch_bounds__(256) seed_grid_kernel(const dev::QueryNodes no
     coarse[i] = make_int4(hit.slot, 0, kEmptyChild, kEmptyChild);
   } else {
     // the coarse lattice is a seed grid itself, each node its nearest point's seed
-    const dev::SeedGrid g{coarse, lox, loy, loz, 1.0f / (h * kSeedStride), n / kSeedStride};
+    const dev::SeedGrid g{coarse, lox, loy, loz, 1.0f / (h * kSeedStride), n / kSeedStride, INFINITY};
     if (ix % kSeedStride == 0 && iy % kSeedStride == 0 && iz % kSeedStride == 0) {
       const int m = n / kSeedStride + 1;
       hit.slot = coarse[(static_cast<int64_t>(iz / kSeedStride) * m + iy / kSeedStride) * m + ix / kSeedStride].x;
@@ -347,7 +363,8 @@ __global__ void __launch_bounds__(64) sample_work_kernel(const dev::QueryNodes n
   seed.id = INT32_MAX;
   seed.slot = -1;
   seed.cp = p;
-  const int4 cell = dev::seed_cell_any(grid, p, 0);
+  bool far;
+  const int4 cell = dev::seed_cell_any(grid, p, 0, far);
   dev::test_slot(tris, cell.x, p, seed);
   uint32_t units[2] = {0, 0};
   bool overflow = false;
@@ -491,6 +508,30 @@ void choose_nodes(n2w_bvh& b, int triangles, const dev::SeedGrid& grid) {
   b.use_boxes = boxes < frames;
 }
 
+// SeedGrid::far.  The margin of the frame nodes' limit (prune_limit) grows with the
+// query's distance d from the mesh c, 2^-20 |p|_1 + 2^-18 d <= 5.3e-6 d + 2^-20 |c|_1.
+// Where it reaches a quarter of the triangles' edge it covers patches of them, and the
+// axis-aligned boxes, which need none, leave far fewer to test: 81,920 triangles, work of
+// a query over frames / boxes 158 / 244 at 500 extents, 1,764 / 249 at 5,000.
+float far_limit(const n2w_bvh& b, const n2w_mesh& mesh) {
+  double edge = 0.0;
+  for (const auto& t : mesh.triangles) {
+    double l2[2] = {0.0, 0.0};
+    for (int a = 0; a < 3; ++a) {
+      const double x = mesh.vertices[t[0]][a];
+      l2[0] += (mesh.vertices[t[1]][a] - x) * (mesh.vertices[t[1]][a] - x);
+      l2[1] += (mesh.vertices[t[2]][a] - x) * (mesh.vertices[t[2]][a] - x);
+    }
+    edge += std::sqrt(std::max(l2[0], l2[1]));
+  }
+  edge /= static_cast<double>(mesh.triangles.size());
+  const double half = 0.5 * b.seed_n * static_cast<double>(b.seed_h);
+  double centre = 0.0;
+  for (int a = 0; a < 3; ++a) centre += std::fabs(b.seed_lo[a] + half);
+  const double far = (0.25 * edge - centre * 0x1p-20) / (5.3e-6 * half);
+  return static_cast<float>(far > 0.0 ? far : 0.0);  // (not a number: 0)
+}
+
 // Seed grid over the mesh box grown by 20 % of its largest extent on every side.
 void build_seed_grid(n2w_bvh& b, const n2w_mesh& mesh, int n) {
   float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -523,7 +564,8 @@ void build_seed_grid(n2w_bvh& b, const n2w_mesh& mesh, int n) {
     N2W_CUDA(cudaGetLastError());
     choose_nodes(b, static_cast<int>(mesh.triangles.size()),
                  dev::SeedGrid{coarse, b.seed_lo[0], b.seed_lo[1], b.seed_lo[2], 1.0f / (h * kSeedStride),
-                               n / kSeedStride});
+                               n / kSeedStride, INFINITY});
+    b.seed_far = far_limit(b, mesh);
     seed_grid_kernel<false><<<static_cast<unsigned>((total + block - 1) / block), block>>>(
         query_nodes_of(b), tris, b.seed_lo[0], b.seed_lo[1], b.seed_lo[2], h, n, coarse, b.d_seed, d_ov);
     N2W_CUDA(cudaGetLastError());

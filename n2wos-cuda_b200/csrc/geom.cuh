@@ -420,7 +420,8 @@ struct SeedGrid {
   const int4* cells;  // nullptr when absent
   float lo_x, lo_y, lo_z;
   float inv_h;
-  int n;  // cells per axis
+  int n;      // cells per axis
+  float far;  // distance from the lattice's centre, in half lattices, from which queries search boxes (far_limit)
 };
 
 // The cell of the lattice node nearest to p; outside the lattice the clamped
@@ -443,22 +444,25 @@ __device__ __forceinline__ int4 seed_cell(const SeedGrid& g, V3 p, int root) {
 // lattice's centre to p leaves it, with the root as its only subtree.  (A point
 // clamped axis by axis lies in another direction from the mesh, and its triangle is
 // a poor seed.)  300,000 queries around 81,920 triangles, 5 extents from their centre:
-// 3,535 -> 869 us, 1.5 extents: 2,017 -> 645 us.
-__device__ __forceinline__ int4 seed_cell_any(const SeedGrid& g, V3 p, int root) {
+// 3,535 -> 869 us, 1.5 extents: 2,017 -> 645 us.  `far`: the margin of the frame nodes'
+// limit at p is large against the triangles (far_limit).
+__device__ __forceinline__ int4 seed_cell_any(const SeedGrid& g, V3 p, int root, bool& far) {
   const float half = 0.5f * static_cast<float>(g.n), n = static_cast<float>(g.n);
   const float fx = (p.x - g.lo_x) * g.inv_h - half, fy = (p.y - g.lo_y) * g.inv_h - half,
               fz = (p.z - g.lo_z) * g.inv_h - half;
-  const float far = fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz)));
+  const float out = fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz)));
   const bool in = fabsf(fx) <= half && fabsf(fy) <= half && fabsf(fz) <= half;
-  const float s = in ? 1.0f : half / far;
+  const float s = in ? 1.0f : half / out;
   // (not a number: node 0)
   const float cx = fminf(fmaxf(fmaf(fx, s, half), 0.0f), n), cy = fminf(fmaxf(fmaf(fy, s, half), 0.0f), n),
               cz = fminf(fmaxf(fmaf(fz, s, half), 0.0f), n);
   const int m = g.n + 1;
   int4 c = __ldg(g.cells + (static_cast<size_t>(__float2int_rn(cz)) * m + __float2int_rn(cy)) * m + __float2int_rn(cx));
+  far = false;
   if (!in) {
     c.y = root;
     c.z = c.w = kEmptyChild;
+    far = out > half * g.far;
   }
   return c;
 }
@@ -784,10 +788,11 @@ __device__ __forceinline__ void traverse_query(const QueryNodes& nodes, const fl
   FrameStack stack;
   FrameTrav t;
   if (grid.cells) {
-    const int4 cell = seed_cell_any(grid, p, root);
+    bool far;
+    const int4 cell = seed_cell_any(grid, p, root, far);
     test_slot(tris, cell.x, p, hit);
     ++st.tri_tests;
-    if (nodes.use_boxes) {
+    if (nodes.use_boxes || far) {
       traverse(nodes.boxes, tris, p, hit, st, root);
       return;
     }

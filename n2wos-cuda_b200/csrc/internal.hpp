@@ -27,6 +27,7 @@ struct n2w_bvh {
   float seed_lo[3] = {0, 0, 0};
   float seed_h = 0.0f;
   int seed_n = 0;
+  float seed_far = 0.0f;   // SeedGrid::far
   bool use_boxes = false;  // queries search d_nodes, not d_frames (choose_nodes)
   n2w_bvh_stats stats{};
   int device = 0;

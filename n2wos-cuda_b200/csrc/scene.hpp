@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <vector>
 
 #include "internal.hpp"
@@ -42,6 +43,7 @@ inline void set_instance_geometry(BatchInst& I, const n2w_scene& sc, int mesh) {
   I.grid.lo_z = m.seed_lo[2];
   I.grid.inv_h = m.seed_h > 0.0f ? 1.0f / m.seed_h : 0.0f;
   I.grid.n = m.seed_n;
+  I.grid.far = INFINITY;  // a scene holds the frames only
   for (int a = 0; a < 3; ++a) {
     I.box_lo[a] = m.box_lo[a];
     I.box_hi[a] = m.box_hi[a];

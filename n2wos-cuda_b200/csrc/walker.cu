@@ -647,7 +647,7 @@ __global__ void __launch_bounds__(256) first_query_kernel(const __grid_constant_
   hit.slot = -1;
   hit.cp = f.p;
   dev::TraversalStats st{0, 0, 0};
-  dev::traverse_query(dev::QueryNodes{a.nodes, a.boxes, a.boxes != nullptr}, a.tris, f.grid, f.p, hit, st, f.root);
+  dev::traverse_query(dev::QueryNodes{a.nodes, a.boxes, a.first_boxes != 0}, a.tris, f.grid, f.p, hit, st, f.root);
   cpd[i] = make_float4(hit.cp.x, hit.cp.y, hit.cp.z, hit.d2);
   ids[i] = make_int2(hit.id, hit.slot);
   if (a.counters) {
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) first_query_warp_ker
   if (i >= n) return;
   const FirstQuery f = first_query_of<kBatch>(a, i);
   const dev::WarpBest b =
-      dev::warp_query(dev::QueryNodes{a.nodes, a.boxes, a.boxes != nullptr}, a.tris, f.grid, f.p, f.root, f.p,
+      dev::warp_query(dev::QueryNodes{a.nodes, a.boxes, a.first_boxes != 0}, a.tris, f.grid, f.p, f.root, f.p,
                       s_work + warp * dev::kWarpList);
   if (b.winner()) {
     cpd[i] = make_float4(b.cp.x, b.cp.y, b.cp.z, dev::key_d2(b.key));
@@ -867,7 +867,8 @@ WalkArgs make_walk_args(const n2w_bvh& bvh, const n2w_problem& problem, const n2
                         int64_t point_count, const n2w_walk_options& o, uint32_t stream_tag) {
   WalkArgs a{};
   a.nodes = reinterpret_cast<const float4*>(bvh.d_frames);
-  a.boxes = bvh.use_boxes ? reinterpret_cast<const float4*>(bvh.d_nodes) : nullptr;
+  a.boxes = reinterpret_cast<const float4*>(bvh.d_nodes);
+  a.first_boxes = bvh.use_boxes ? 1 : 0;
   a.tris = reinterpret_cast<const float4*>(bvh.d_edges);
   a.grid = seed_grid_of(bvh);
   for (int k = 0; k < 3; ++k) {

@@ -60,7 +60,7 @@ struct alignas(16) BatchInst {
 
 struct WalkArgs {
   const float4* nodes;  // FrameNode4 array
-  const float4* boxes;  // Node4 array of the same tree if its first queries search that, else nullptr
+  const float4* boxes;  // Node4 array of the same tree, for first queries (batched launches: nullptr)
   const float4* tris;   // TriEdges array
   dev::SeedGrid grid;
   float box_lo[3], box_hi[3];  // domain box: the mesh box grown by 20 % (walks never leave it)
@@ -83,6 +83,7 @@ struct WalkArgs {
   int has_source;
   int source_center;
   int source_samples;  // points averaged per ball (>= 1)
+  int first_boxes;     // first queries search `boxes` (n2w_bvh::use_boxes)
   int64_t deadline_ns;
   n2w_problem problem;
   // kOutStats

@@ -134,8 +134,8 @@ __device__ __forceinline__ void warp_search_over(const float4* __restrict__ node
 }
 
 __device__ __forceinline__ void warp_search(const QueryNodes& nodes, const float4* __restrict__ tris, V3 p, int4 start,
-                                            WarpBest& b, int2* work) {
-  if (nodes.use_boxes) warp_search_over<true>(nodes.boxes, tris, p, start, b, work);
+                                            bool far, WarpBest& b, int2* work) {
+  if (nodes.use_boxes || far) warp_search_over<true>(nodes.boxes, tris, p, start, b, work);
   else warp_search_over<false>(nodes.frames, tris, p, start, b, work);
 }
 
@@ -148,15 +148,16 @@ __device__ __forceinline__ WarpBest warp_query(const QueryNodes& nodes, const fl
   h.slot = -1;
   h.cp = no_hit;
   int4 cell = make_int4(0, root, kEmptyChild, kEmptyChild);
+  bool far = false;
   if (grid.cells) {
-    cell = seed_cell_any(grid, p, root);
+    cell = seed_cell_any(grid, p, root, far);
     test_slot(tris, cell.x, p, h);
   }
   WarpBest b;
   b.key = b.mine = hit_key(h.d2, h.id);
   b.cp = h.cp;
   b.slot = h.slot;
-  warp_search(nodes, tris, p, cell, b, work);
+  warp_search(nodes, tris, p, cell, far, b, work);
   if (grid.cells && (threadIdx.x & 31) == 0) ++b.tris;
   return b;
 }

@@ -111,3 +111,35 @@ def test_trees_whose_frames_do_not_pay(gpu, request, name, where, n):
     assert_same_answers(bvh.query(pts), want)
     if n > SWITCH:
         assert first_query_work(gpu, bvh, pts) <= 1.0 * (want["node_visits"] + want["tri_tests"]).mean()
+
+
+@pytest.mark.parametrize("extents,offset", [(5e3, 0.0), (5e4, 0.0), (0.5, 2e4), (50.0, 1e3)])
+def test_far_coordinates_search_the_boxes(gpu, sphere, extents, offset):
+    """Thousands of extents away, or with the mesh that far from the origin, the framed nodes' rounding margin covers
+    whole patches; the search then does no more work than the counted query."""
+    bvh, v = sphere
+    if offset:
+        _, t = gpu.Mesh.icosphere_displaced(5, 0.12, 3.0, 4, 0.5, 12345).arrays()
+        v = v + np.float32(offset)
+        bvh = gpu.Bvh(gpu.Mesh.from_arrays(v, t), 4, "sah")
+    pts = sphere_points(v, SWITCH + 37, extents, 5)
+    want = bvh.query(pts, counted=True)
+    assert_same_answers(bvh.query(pts), want)
+    assert_same_answers(bvh.query(pts[:1000]), {k: x[:1000] for k, x in want.items()})
+    counted = (want["node_visits"] + want["tri_tests"]).mean()
+    assert first_query_work(gpu, bvh, pts) <= 1.0 * counted
+
+
+def test_few_far_points_among_near_ones(gpu, sphere):
+    """Far points scattered through a launch of near ones, and whole warps of them: handed off at once, the rest not."""
+    bvh, v = sphere
+    rng = np.random.default_rng(8)
+    pts = rng.uniform(-1.2, 1.2, (SWITCH + 37, 3)).astype(np.float32)
+    far = sphere_points(v, len(pts), 5e3, 9)
+    sel = np.zeros(len(pts), bool)
+    sel[::41] = True  # less than one a warp
+    sel[10_000:10_000 + 100] = True  # whole warps, from the middle of one
+    sel[-3:] = True
+    pts[sel] = far[sel]
+    want = bvh.query(pts, counted=True)
+    assert_same_answers(bvh.query(pts), want)
