@@ -79,21 +79,20 @@ constexpr int kQueryBlocks = 4;
 enum { kFrames, kBoxes, kCounted };  // frame nodes; boxes; boxes with every visit from the root counted
 
 // One lane's query in flight; step() returns false once it is complete.
-template <int kMode>
+template <int kMode, bool kL1>
 struct Search {
   dev::TravState t;
   int2 stack[kTraversalStack];
   __device__ __forceinline__ void start(int4) { t = dev::TravState{0, 0, 0, 0}; }
   __device__ __forceinline__ bool step(const float4* __restrict__ nodes, const float4* __restrict__ tris, dev::V3 p,
                                        dev::ClosestHit& hit, uint32_t& c_nodes, uint32_t& c_tris, bool& overflow) {
-    // Two units per pass.  Few nodes are visited here and often the same, so the loads
-    // keep their L1 lines.
-    return dev::trav_step_boxes<true>(nodes, tris, p, hit, t, stack, c_nodes, c_tris, overflow) &&
-           (kMode == kCounted || dev::trav_step_boxes<true>(nodes, tris, p, hit, t, stack, c_nodes, c_tris, overflow));
+    // Two units per pass.
+    return dev::trav_step_boxes<kL1>(nodes, tris, p, hit, t, stack, c_nodes, c_tris, overflow) &&
+           (kMode == kCounted || dev::trav_step_boxes<kL1>(nodes, tris, p, hit, t, stack, c_nodes, c_tris, overflow));
   }
 };
-template <>
-struct Search<kFrames> {
+template <bool kL1>
+struct Search<kFrames, kL1> {
   dev::FrameTrav t;
   dev::FrameStack stack;
   __device__ __forceinline__ void start(int4 cell) { t.start(cell, stack); }
@@ -102,14 +101,14 @@ struct Search<kFrames> {
     // Two nodes per triangle: uniform queries expand 26 nodes and test 13
     // triangles (one node: 372 against 357 us for 262,144 queries, equal for
     // 1,000,003 near the surface and 4,194,304).
-    dev::trav_triangle<false>(tris, p, hit, t, stack, c_tris);
-    dev::trav_node<false, true>(frames, p, hit, t, stack, c_nodes, overflow);
-    dev::trav_node<false, true>(frames, p, hit, t, stack, c_nodes, overflow);
+    dev::trav_triangle<false, kL1>(tris, p, hit, t, stack, c_tris);
+    dev::trav_node<kL1, true>(frames, p, hit, t, stack, c_nodes, overflow);
+    dev::trav_node<kL1, true>(frames, p, hit, t, stack, c_nodes, overflow);
     return !t.done();
   }
 };
 
-template <bool kMasked, int kMode>
+template <bool kMasked, int kMode, bool kL1>
 __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kernel(
     const float4* __restrict__ nodes, const float4* __restrict__ tris, const dev::SeedGrid grid,
     const n2w_vec3* __restrict__ points, const uint8_t* __restrict__ active, int n,
@@ -132,7 +131,7 @@ __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kerne
   hit.cp = p;
   uint32_t c_nodes = 0, c_tris = 0;
   bool overflow = false;
-  Search<kMode> search;
+  Search<kMode, kL1> search;
   // Hands the query to the finisher with its best so far (a bound on the answer) in
   // its own output slots.
   auto hand_off = [&](int mark) {
@@ -172,7 +171,7 @@ __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kerne
       if (grid.cells) {
         bool far = false;
         cell = kCount ? dev::seed_cell(grid, p, 0) : dev::seed_cell_any(grid, p, 0, far);
-        dev::test_slot(tris, cell.x, p, hit);
+        dev::test_slot<kL1>(tris, cell.x, p, hit);
         ++c_tris;
         if (kMode == kFrames && far) {
           hand_off(kHandOffFar);
@@ -370,7 +369,7 @@ __global__ void __launch_bounds__(64) sample_work_kernel(const dev::QueryNodes n
   bool overflow = false;
   {
     dev::ClosestHit hit = seed;
-    Search<kFrames> s;
+    Search<kFrames, true> s;
     uint32_t c_nodes = 0, c_tris = 0;
     s.start(cell);
     while (!s.t.done() && c_nodes + c_tris < kSampleUnits) {
@@ -380,7 +379,7 @@ __global__ void __launch_bounds__(64) sample_work_kernel(const dev::QueryNodes n
   }
   {
     dev::ClosestHit hit = seed;
-    Search<kBoxes> s;
+    Search<kBoxes, true> s;
     uint32_t c_nodes = 0, c_tris = 0;
     s.start(cell);
     while (c_nodes + c_tris < kSampleUnits && s.step(nodes.boxes, tris, p, hit, c_nodes, c_tris, overflow)) {
@@ -445,7 +444,7 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
   if (d_nodes) {
     // the counting variant runs every query to completion in one lane, so its
     // counts are the single-lane traversal's (the algorithmic work)
-    launch(closest_point_kernel<false, kCounted>, nodes.boxes, d_active, 0, d_nodes, d_tris);
+    launch(closest_point_kernel<false, kCounted, true>, nodes.boxes, d_active, 0, d_nodes, d_tris);
     N2W_CUDA(cudaGetLastError());
     return;
   }
@@ -458,10 +457,14 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
     return;
   }
   if (nodes.use_boxes) {
-    auto kern = d_active ? closest_point_kernel<true, kBoxes> : closest_point_kernel<false, kBoxes>;
+    // few nodes are visited, and often the same: their lines are kept
+    auto kern = d_active ? closest_point_kernel<true, kBoxes, true> : closest_point_kernel<false, kBoxes, true>;
     launch(kern, nodes.boxes, d_active, kBoxBudget, nullptr, nullptr);
+  } else if (fits_l1(bvh.stats.nodes, bvh.stats.triangles)) {
+    auto kern = d_active ? closest_point_kernel<true, kFrames, true> : closest_point_kernel<false, kFrames, true>;
+    launch(kern, nodes.frames, d_active, kQueryBudget, nullptr, nullptr);
   } else {
-    auto kern = d_active ? closest_point_kernel<true, kFrames> : closest_point_kernel<false, kFrames>;
+    auto kern = d_active ? closest_point_kernel<true, kFrames, false> : closest_point_kernel<false, kFrames, false>;
     launch(kern, nodes.frames, d_active, kQueryBudget, nullptr, nullptr);
   }
   N2W_CUDA(cudaGetLastError());

@@ -185,8 +185,8 @@ __device__ __forceinline__ void cswap(float& da, int& ra, float& db, int& rb) {
 // the lanes' lists.  262,144 / 4,194,304 uniform queries 391 -> 374 us / 4.77 ->
 // 4.37 ms, Laplace / Poisson walks 17.4 -> 16.0 / 46.1 -> 43.4 ms, batched
 // instances 37.3 -> 33.8 ms (evict_first: 17.1 / 45.0 / 36.4; evict_last: as
-// without a hint).  kL1 keeps the allocation for launches of few walkers per
-// SM, whose nodes do fit.
+// without a hint).  kL1 keeps the allocation where most loads do hit: launches of
+// few walkers per SM, small trees (fits_l1) and the axis-aligned boxes.
 template <bool kL1 = false>
 __device__ __forceinline__ void ldg_v8f(const float4* p, float4& a, float4& b) {
   if constexpr (kL1) {
@@ -401,8 +401,9 @@ template <bool kFast, bool kL1 = false>
 __device__ __forceinline__ void test_slot_impl(const float4* __restrict__ tris, int slot, V3 p, ClosestHit& hit) {
   test_rec<kFast>(load_rec<kL1>(tris, slot), slot, p, hit);
 }
+template <bool kL1 = false>
 __device__ __forceinline__ void test_slot(const float4* __restrict__ tris, int slot, V3 p, ClosestHit& hit) {
-  test_slot_impl<false>(tris, slot, p, hit);
+  test_slot_impl<false, kL1>(tris, slot, p, hit);
 }
 template <bool kL1>
 __device__ __forceinline__ void test_slot_fast(const float4* __restrict__ tris, int slot, V3 p, ClosestHit& hit) {

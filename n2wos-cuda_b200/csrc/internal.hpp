@@ -111,6 +111,17 @@ void copy_cell_slots(const n2w_bvh& b, int64_t n, int* out);
 
 void build_seed_grid(n2w_bvh& b, const n2w_mesh& mesh, int n);
 
+// Whether a tree's frame nodes and triangles are few enough that most of a launch's loads
+// hit in L1 (256 KB per SM, shared with the lanes' lists) if they allocate there.
+// 1,000,003 uniform queries with / without: 80 triangles 376 / 793 us, 1,280 (125 KB)
+// 545 / 730, 3,000 in a soup (320 KB) 294 / 404, 5,120 (500 KB) 705 / 759, 20,480 in a
+// smooth mesh 950 / 909; 12 triangles 69 / 193.  20,000 x 256 walks 11.8 / 22.9, 17.5 / 20.2,
+// 39.4 / 57.6, 23.7 / 22.8 ms on the first four (3,968 triangles, 340 KB: 21.5 / 21.0).
+constexpr int64_t kL1Bytes = 288 << 10;
+inline bool fits_l1(int64_t nodes, int64_t triangles) {
+  return nodes * static_cast<int64_t>(sizeof(FrameNode4)) + triangles * static_cast<int64_t>(sizeof(TriEdges)) <= kL1Bytes;
+}
+
 void launch_inside(const n2w_bvh& bvh, const n2w_vec3* d_points, int n, uint8_t* d_inside, int* d_overflow,
                    int block_size, cudaStream_t stream);
 

@@ -556,6 +556,7 @@ TickWork tick_launch(n2w_server& s) {
   WalkArgs a{};
   a.nodes = reinterpret_cast<const float4*>(s.scene->d_nodes);
   a.tris = reinterpret_cast<const float4*>(s.scene->d_tris);
+  a.small_tree = fits_l1(s.scene->nodes, s.scene->tris) ? 1 : 0;
   a.first_cpd = s.d_cpd;
   a.first_ids = s.d_ids;
   a.total_chunks = cbase;

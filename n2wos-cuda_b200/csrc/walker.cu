@@ -257,7 +257,8 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 //    warp returns to Phase A once `regen` lanes are waiting (or none is busy),
 //    so the walk updates run for many lanes at once and no lane waits for
 //    another lane's whole traversal.
-template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks, bool kL1 = false>
+//  kL1: nodes and triangles keep L1 lines.  kBoth: a step loads both its records first.
+template <int kOut, int kWalk, bool kBatch, int kMinBlocks, bool kL1, bool kBoth>
 __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(const __grid_constant__ WalkArgs a) {
   static_assert(!kBatch || (kOut == kOutStats && kWalk == N2W_WALK_PURE),
                 "batched launches run plain walks into per-point statistics");
@@ -564,11 +565,11 @@ __global__ void __launch_bounds__(kWalkerMaxThreads, kMinBlocks) walker_kernel(c
       if (busy == 0 || __popc(waiting) >= a.regen) break;
       if (querying) {
         bool ov = false;
-        if constexpr (kL1) {
+        if constexpr (kBoth) {
           dev::trav_both<true, kL1>(a.nodes, a.tris, x, hit, tv, stack, c_nodes, c_tris, ov);
         } else {
-          dev::trav_triangle<true>(a.tris, x, hit, tv, stack, c_tris);
-          dev::trav_node(a.nodes, x, hit, tv, stack, c_nodes, ov);
+          dev::trav_triangle<true, kL1>(a.tris, x, hit, tv, stack, c_tris);
+          dev::trav_node<kL1>(a.nodes, x, hit, tv, stack, c_nodes, ov);
         }
         querying = !tv.done();
         if (ov) {
@@ -760,9 +761,9 @@ namespace {
 constexpr int kSpreadWarps = 16;
 constexpr int kSpreadMinBlocks = 2;
 
-template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinBlocks, bool kL1 = false>
+template <int kOut, int kWalk, bool kBatch, int kMinBlocks, bool kL1, bool kBoth>
 void launch_walker_kernel(WalkArgs a, int block, int blocks_per_sm, cudaStream_t stream) {
-  auto kern = walker_kernel<kOut, kWalk, kBatch, kMinBlocks, kL1>;
+  auto kern = walker_kernel<kOut, kWalk, kBatch, kMinBlocks, kL1, kBoth>;
   int occ = 0;
   N2W_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, block, 0));
   if (occ < 1) occ = 1;
@@ -785,10 +786,13 @@ void launch_walker(WalkArgs a, int block, int blocks_per_sm, cudaStream_t stream
     if (lanes < 32) {
       a.lanes = static_cast<int>(lanes);
       a.regen = std::max(1, a.regen * a.lanes / 32);
-      return launch_walker_kernel<kOut, kWalk, kBatch, kSpreadMinBlocks, true>(a, block, blocks_per_sm, stream);
+      return launch_walker_kernel<kOut, kWalk, kBatch, kSpreadMinBlocks, true, true>(a, block, blocks_per_sm, stream);
     }
   }
-  launch_walker_kernel<kOut, kWalk, kBatch, kMinBlocks>(a, block, blocks_per_sm, stream);
+  // Small trees keep their L1 lines (fits_l1): 40,000 points x 16 walks, 12 triangles
+  // 3,392 -> 1,033 us.
+  if (a.small_tree) launch_walker_kernel<kOut, kWalk, kBatch, kMinBlocks, true, false>(a, block, blocks_per_sm, stream);
+  else launch_walker_kernel<kOut, kWalk, kBatch, kMinBlocks, false, false>(a, block, blocks_per_sm, stream);
 }
 
 // First queries of n points; up to kWarpPoints points a warp each, else a lane
@@ -828,11 +832,11 @@ void launch_walker_batch(const WalkArgs& a, int block, int blocks_per_sm, int re
 int walker_batch_occupancy(int block, int reg_variant) {
   int occ = 0;
   if (reg_variant == 1) {
-    N2W_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, walker_kernel<kOutStats, N2W_WALK_PURE, true, 3>,
-                                                            block, 0));
+    N2W_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &occ, walker_kernel<kOutStats, N2W_WALK_PURE, true, 3, false, false>, block, 0));
   } else {
-    N2W_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, walker_kernel<kOutStats, N2W_WALK_PURE, true, 4>,
-                                                            block, 0));
+    N2W_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &occ, walker_kernel<kOutStats, N2W_WALK_PURE, true, 4, false, false>, block, 0));
   }
   return occ;
 }
@@ -869,6 +873,7 @@ WalkArgs make_walk_args(const n2w_bvh& bvh, const n2w_problem& problem, const n2
   a.nodes = reinterpret_cast<const float4*>(bvh.d_frames);
   a.boxes = reinterpret_cast<const float4*>(bvh.d_nodes);
   a.first_boxes = bvh.use_boxes ? 1 : 0;
+  a.small_tree = fits_l1(bvh.stats.nodes, bvh.stats.triangles) ? 1 : 0;
   a.tris = reinterpret_cast<const float4*>(bvh.d_edges);
   a.grid = seed_grid_of(bvh);
   for (int k = 0; k < 3; ++k) {

@@ -1,0 +1,63 @@
+"""Launches that must not cost more than comparable ones: device times of pairs of
+calls on one GPU, medians of interleaved runs, with wide bounds."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def timed_in_turn(gpu, calls, repeat=9):
+    """Median device milliseconds of each call, run in turn."""
+    stream, timer = gpu.Stream(), gpu.Timer()
+    ms = [[] for _ in calls]
+    for r in range(repeat + 2):
+        for c, out in zip(calls, ms):
+            timer.start(stream)
+            c(stream)
+            timer.stop(stream)
+            t = timer.ms()
+            if r >= 2:  # two rounds of warm-up
+                out.append(t)
+    return [float(np.median(x)) for x in ms]
+
+
+def query_call(gpu, bvh, pts):
+    n = len(pts)
+    b = gpu.DeviceBuffer
+    p, d2, cp, ids, ov = b.from_array(pts), b(4 * n), b(12 * n), b(4 * n), b(4 * n)
+    return lambda s: bvh.query_device(p.ptr, n, d2.ptr, cp.ptr, ids.ptr, ov.ptr, 128, s)
+
+
+def walk_call(gpu, bvh, pts, **options):
+    from n2w._lib import call
+
+    n = len(pts)
+    p, st = gpu.DeviceBuffer.from_array(pts), gpu.PointStatsBuffers.allocate(n)
+    o = gpu.walk_options(max_steps=256, epsilon=1e-3, **options)
+    pb = gpu.problem_charges_seeded(8, 1.6, 2.0, 12345)
+    return lambda s: call("n2w_wos_estimate", bvh.handle, C.byref(pb), p.ptr, n, C.byref(o), st.struct(), None, None,
+                          s.handle)
+
+
+def icosphere(gpu, level):
+    m = gpu.Mesh.icosphere_displaced(level, 0.12, 3.0, 4, 0.5, 12345)
+    m.normalize()
+    return gpu.Bvh(m, 4, "sah")
+
+
+@pytest.fixture(scope="module")
+def small_and_large(gpu):
+    return icosphere(gpu, 1), icosphere(gpu, 6)
+
+
+def test_small_trees_stay_in_l1(gpu, small_and_large):
+    """80 triangles (7 KB of nodes and triangles) against 81,920: the same queries take much less, the same walks too."""
+    rng = np.random.default_rng(2)
+    pts = rng.uniform(-1.2, 1.2, (1_000_003, 3)).astype(np.float32)
+    small, large = timed_in_turn(gpu, [query_call(gpu, b, pts) for b in small_and_large])
+    assert small < 0.65 * large, (small, large)
+    pts = rng.uniform(-0.3, 0.3, (20_000, 3)).astype(np.float32)
+    small, large = timed_in_turn(gpu, [walk_call(gpu, b, pts, walks_per_point=128) for b in small_and_large], 5)
+    assert small < 0.65 * large, (small, large)
