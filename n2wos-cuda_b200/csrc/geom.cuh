@@ -448,22 +448,25 @@ __device__ __forceinline__ int4 seed_cell(const SeedGrid& g, V3 p, int root) {
 // 3,535 -> 869 us, 1.5 extents: 2,017 -> 645 us.  `far`: the margin of the frame nodes'
 // limit at p is large against the triangles (far_limit).
 __device__ __forceinline__ int4 seed_cell_any(const SeedGrid& g, V3 p, int root, bool& far) {
-  const float half = 0.5f * static_cast<float>(g.n), n = static_cast<float>(g.n);
-  const float fx = (p.x - g.lo_x) * g.inv_h - half, fy = (p.y - g.lo_y) * g.inv_h - half,
-              fz = (p.z - g.lo_z) * g.inv_h - half;
-  const float out = fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz)));
-  const bool in = fabsf(fx) <= half && fabsf(fy) <= half && fabsf(fz) <= half;
-  const float s = in ? 1.0f : half / out;
-  // (not a number: node 0)
-  const float cx = fminf(fmaxf(fmaf(fx, s, half), 0.0f), n), cy = fminf(fmaxf(fmaf(fy, s, half), 0.0f), n),
-              cz = fminf(fmaxf(fmaf(fz, s, half), 0.0f), n);
+  const float fx = (p.x - g.lo_x) * g.inv_h, fy = (p.y - g.lo_y) * g.inv_h, fz = (p.z - g.lo_z) * g.inv_h;
+  const float n = static_cast<float>(g.n), half = 0.5f * n;
+  float cx = fminf(fmaxf(fx, 0.0f), n), cy = fminf(fmaxf(fy, 0.0f), n), cz = fminf(fmaxf(fz, 0.0f), n);
+  const bool in = cx == fx && cy == fy && cz == fz;
+  far = false;
+  if (!in) {
+    const float dx = fx - half, dy = fy - half, dz = fz - half;
+    const float out = fmaxf(fabsf(dx), fmaxf(fabsf(dy), fabsf(dz)));
+    const float s = half / out;
+    cx = fminf(fmaxf(fmaf(dx, s, half), 0.0f), n);  // (not a number: node 0)
+    cy = fminf(fmaxf(fmaf(dy, s, half), 0.0f), n);
+    cz = fminf(fmaxf(fmaf(dz, s, half), 0.0f), n);
+    far = out > half * g.far;
+  }
   const int m = g.n + 1;
   int4 c = __ldg(g.cells + (static_cast<size_t>(__float2int_rn(cz)) * m + __float2int_rn(cy)) * m + __float2int_rn(cx));
-  far = false;
   if (!in) {
     c.y = root;
     c.z = c.w = kEmptyChild;
-    far = out > half * g.far;
   }
   return c;
 }
