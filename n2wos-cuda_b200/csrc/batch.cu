@@ -153,6 +153,7 @@ WalkArgs batch_args(const n2w_batch& b, n2w_walk_counters* d_counters) {
   a.nodes = reinterpret_cast<const float4*>(b.scene->d_nodes);
   a.tris = reinterpret_cast<const float4*>(b.scene->d_tris);
   a.small_tree = fits_l1(b.scene->nodes, b.scene->tris) ? 1 : 0;
+  a.warp_points = warp_query_limit(b.scene->tris, false, true);
   a.first_cpd = b.d_cpd;
   a.first_ids = b.d_ids;
   a.total_chunks = b.total_chunks;

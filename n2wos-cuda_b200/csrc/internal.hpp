@@ -95,6 +95,19 @@ struct HostBvh {
 HostBvh build_bvh4(const n2w_mesh& mesh, int leaf_size, const std::string& method);
 n2w_bvh_stats host_stats(const HostBvh& h, int leaf_size, double ms);
 
+// Launches of up to this many queries (or first queries of walks) give each a warp: with
+// a lane per query a launch lasts as long as its slowest serial search, whatever its size,
+// but a warp per query takes longer for queries that are short.  Lane / warp per query over
+// the frames of 81,920 triangles: 8,000 uniform 128 / 32 us, 16,000 124 / 61, 32,768
+// 140 / 99; near the surface 33 / 23, 35 / 39, 38 / 70.  Boxes, whose search wants an order
+// that a warp's batches do not have, near an axis-aligned cube: 8,000 20 / 21, 16,000
+// 21 / 32.  12 triangles: 8,000 around them 14 / 25.
+// First queries over frames keep to warps for longer: their lanes have no budget to hand a
+// long search off by (24,000 in a bumpy sphere of 65,024 triangles: 236 / 120 us).
+inline int warp_query_limit(int64_t triangles, bool boxes, bool first_queries) {
+  return triangles <= 32 ? 4096 : (boxes ? 8192 : (first_queries ? 32768 : 16384));
+}
+
 // ---- device query launch (closest_point.cu) ----
 void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const uint8_t* d_active,
                           int n, float* d_d2, n2w_vec3* d_cp, int* d_id, int* d_overflow,

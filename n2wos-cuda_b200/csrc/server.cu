@@ -557,6 +557,7 @@ TickWork tick_launch(n2w_server& s) {
   a.nodes = reinterpret_cast<const float4*>(s.scene->d_nodes);
   a.tris = reinterpret_cast<const float4*>(s.scene->d_tris);
   a.small_tree = fits_l1(s.scene->nodes, s.scene->tris) ? 1 : 0;
+  a.warp_points = warp_query_limit(s.scene->tris, false, true);
   a.first_cpd = s.d_cpd;
   a.first_ids = s.d_ids;
   a.total_chunks = cbase;

@@ -795,15 +795,10 @@ void launch_walker(WalkArgs a, int block, int blocks_per_sm, cudaStream_t stream
   else launch_walker_kernel<kOut, kWalk, kBatch, kMinBlocks, false, false>(a, block, blocks_per_sm, stream);
 }
 
-// First queries of n points; up to kWarpPoints points a warp each, else a lane
-// each.  One short walk per point, lane / warp per first query: 294 / 234 us (40
-// points), 370 / 270 (1,000), 458 / 367 (8,000), 481 / 417 (16,000), 567 / 564
-// (32,000).
-constexpr int64_t kWarpPoints = 32768;
-
+// First queries of n points; up to a.warp_points of them a warp each, else a lane each.
 template <bool kBatch>
 void launch_first_query(const WalkArgs& a, int64_t n, float4* cpd, int2* ids, cudaStream_t s) {
-  if (n <= kWarpPoints) {
+  if (n <= a.warp_points) {
     const unsigned blocks = static_cast<unsigned>((n + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock);
     first_query_warp_kernel<kBatch><<<blocks, 32 * dev::kWarpsPerBlock, dev::kWarpSearchBytes, s>>>(a, n, cpd, ids);
   } else {
@@ -874,6 +869,7 @@ WalkArgs make_walk_args(const n2w_bvh& bvh, const n2w_problem& problem, const n2
   a.boxes = reinterpret_cast<const float4*>(bvh.d_nodes);
   a.first_boxes = bvh.use_boxes ? 1 : 0;
   a.small_tree = fits_l1(bvh.stats.nodes, bvh.stats.triangles) ? 1 : 0;
+  a.warp_points = warp_query_limit(bvh.stats.triangles, bvh.use_boxes, true);
   a.tris = reinterpret_cast<const float4*>(bvh.d_edges);
   a.grid = seed_grid_of(bvh);
   for (int k = 0; k < 3; ++k) {

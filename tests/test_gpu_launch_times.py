@@ -61,3 +61,16 @@ def test_small_trees_stay_in_l1(gpu, small_and_large):
     pts = rng.uniform(-0.3, 0.3, (20_000, 3)).astype(np.float32)
     small, large = timed_in_turn(gpu, [walk_call(gpu, b, pts, walks_per_point=128) for b in small_and_large], 5)
     assert small < 0.65 * large, (small, large)
+
+
+def test_short_queries_in_small_launches(gpu, small_and_large):
+    """Queries close to the surface are short: 32,768 of them, the last size of the small launches' rules, take no more
+    than 1.6 times what one query more takes."""
+    m = gpu.Mesh.icosphere_displaced(6, 0.12, 3.0, 4, 0.5, 12345)
+    m.normalize()
+    v, t = m.arrays()
+    rng = np.random.default_rng(3)
+    tri = v[t[rng.integers(0, len(t), 32769)]]
+    pts = (tri.mean(1) + rng.normal(size=(32769, 3)) * 3e-4).astype(np.float32)
+    small, large = timed_in_turn(gpu, [query_call(gpu, small_and_large[1], p) for p in (pts[:-1], pts)])
+    assert small < 1.6 * large, (small, large)
