@@ -761,15 +761,19 @@ namespace {
 constexpr int kSpreadWarps = 16;
 constexpr int kSpreadMinBlocks = 2;
 
-template <int kOut, int kWalk, bool kBatch, int kMinBlocks, bool kL1, bool kBoth>
-void launch_walker_kernel(WalkArgs a, int block, int blocks_per_sm, cudaStream_t stream) {
-  auto kern = walker_kernel<kOut, kWalk, kBatch, kMinBlocks, kL1, kBoth>;
+// Blocks of a kernel that a launch may keep on an SM.
+template <class Kernel>
+int blocks_on_sm(Kernel kern, int block, int blocks_per_sm) {
   int occ = 0;
   N2W_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, block, 0));
   if (occ < 1) occ = 1;
-  const int per_sm = blocks_per_sm > 0 ? std::min(blocks_per_sm, occ) : occ;
-  const int64_t sms = sm_count_current();
-  int64_t grid = sms * per_sm;
+  return blocks_per_sm > 0 ? std::min(blocks_per_sm, occ) : occ;
+}
+
+template <int kOut, int kWalk, bool kBatch, int kMinBlocks, bool kL1, bool kBoth>
+void launch_walker_kernel(WalkArgs a, int block, int blocks_per_sm, cudaStream_t stream) {
+  auto kern = walker_kernel<kOut, kWalk, kBatch, kMinBlocks, kL1, kBoth>;
+  int64_t grid = static_cast<int64_t>(sm_count_current()) * blocks_on_sm(kern, block, blocks_per_sm);
   const int64_t per_block = static_cast<int64_t>(block / 32) * a.lanes;
   grid = std::min<int64_t>(grid, (a.total_chunks + per_block - 1) / per_block);
   grid = std::max<int64_t>(grid, 1);
@@ -781,11 +785,15 @@ template <int kOut, int kWalk, bool kBatch = false, int kMinBlocks = kWalkerMinB
 void launch_walker(WalkArgs a, int block, int blocks_per_sm, cudaStream_t stream) {
   a.lanes = 32;
   if constexpr (!kBatch) {
-    const int64_t warps = static_cast<int64_t>(sm_count_current()) * kSpreadWarps;
-    const int64_t lanes = (a.total_chunks + warps - 1) / warps;
-    if (lanes < 32) {
-      a.lanes = static_cast<int>(lanes);
-      a.regen = std::max(1, a.regen * a.lanes / 32);
+    const int64_t sms = sm_count_current();
+    if (a.total_chunks <= 31 * sms * kSpreadWarps) {
+      // the warps that the caller's block size and blocks per SM leave
+      const int on_sm = blocks_on_sm(walker_kernel<kOut, kWalk, kBatch, kSpreadMinBlocks, true, true>, block,
+                                     blocks_per_sm) * (block / 32);
+      const int64_t warps = sms * std::min(kSpreadWarps, on_sm);
+      a.lanes = static_cast<int>(std::min<int64_t>((a.total_chunks + warps - 1) / warps, 32));
+      // the default threshold's share of the lanes; the caller's own is a number of lanes
+      a.regen = a.own_regen ? std::min(a.regen, a.lanes) : std::max(1, a.regen * a.lanes / 32);
       return launch_walker_kernel<kOut, kWalk, kBatch, kSpreadMinBlocks, true, true>(a, block, blocks_per_sm, stream);
     }
   }
@@ -881,6 +889,7 @@ WalkArgs make_walk_args(const n2w_bvh& bvh, const n2w_problem& problem, const n2
   a.chunk = o.chunk > 0 ? std::min(o.chunk, o.walks_per_point) : std::min(kDefaultChunk, o.walks_per_point);
   a.chunks_per_point = (o.walks_per_point + a.chunk - 1) / a.chunk;
   a.regen = o.regen_threshold > 0 ? o.regen_threshold : kDefaultRegen;
+  a.own_regen = o.regen_threshold > 0 ? 1 : 0;
   a.total_chunks = point_count * a.chunks_per_point;
   a.max_steps = o.max_steps;
   a.depth_m = o.depth_m;

@@ -85,6 +85,7 @@ struct WalkArgs {
   int source_samples;  // points averaged per ball (>= 1)
   int first_boxes;     // first queries search `boxes` (n2w_bvh::use_boxes)
   int small_tree;      // nodes and triangles stay in L1 (fits_l1)
+  int own_regen;       // regen is the caller's
   int warp_points;     // first queries of up to this many points run one to a warp (warp_query_limit)
   int64_t deadline_ns;
   n2w_problem problem;

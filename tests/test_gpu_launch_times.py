@@ -74,3 +74,12 @@ def test_short_queries_in_small_launches(gpu, small_and_large):
     pts = (tri.mean(1) + rng.normal(size=(32769, 3)) * 3e-4).astype(np.float32)
     small, large = timed_in_turn(gpu, [query_call(gpu, small_and_large[1], p) for p in (pts[:-1], pts)])
     assert small < 1.6 * large, (small, large)
+
+
+def test_few_walks_share_the_warps_that_the_caller_leaves(gpu, small_and_large):
+    """150 x 16 walks in one warp per SM, half as many lanes as it has, take no more than twice what they take with the
+    default launch shape, where each has a warp of its own."""
+    pts = np.random.default_rng(4).uniform(-0.3, 0.3, (150, 3)).astype(np.float32)
+    limited, free = timed_in_turn(gpu, [walk_call(gpu, small_and_large[1], pts, walks_per_point=16, **o) for o in
+                                        (dict(blocks_per_sm=1, block_size=32), {})])
+    assert limited < 2.0 * free, (limited, free)
