@@ -17,6 +17,9 @@
 // too far for a frame to matter, so they keep the axes and the boxes they have.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <vector>
+
 #include "geom.cuh"
 #include "internal.hpp"
 
@@ -281,12 +284,6 @@ __global__ void __launch_bounds__(256) edges_kernel(const TriRec* __restrict__ t
   out[i] = o;
 }
 
-__global__ void __launch_bounds__(256) cell_slots_kernel(const int4* __restrict__ cells, int64_t n,
-                                                         int* __restrict__ slots) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) slots[i] = cells[i].x;
-}
-
 }  // namespace
 
 void build_cell_entries(n2w_bvh& b) {
@@ -297,15 +294,16 @@ void build_cell_entries(n2w_bvh& b) {
   N2W_CUDA(cudaGetLastError());
 }
 
+// Plain copies of whole cells: the BVH may be on another device than the current one,
+// and the device may have no memory left.
 void copy_cell_slots(const n2w_bvh& b, int64_t n, int* out) {
-  int* d = nullptr;
-  N2W_CUDA(cudaMalloc(&d, sizeof(int) * static_cast<size_t>(n)));
-  cell_slots_kernel<<<static_cast<unsigned>((n + 255) / 256), 256>>>(b.d_seed, n, d);
-  const cudaError_t l = cudaGetLastError();
-  const cudaError_t e = cudaMemcpy(out, d, sizeof(int) * static_cast<size_t>(n), cudaMemcpyDeviceToHost);
-  cudaFree(d);
-  N2W_CUDA(l);
-  N2W_CUDA(e);
+  constexpr int64_t kChunk = 1 << 17;
+  std::vector<int4> cells(static_cast<size_t>(std::min(n, kChunk)));
+  for (int64_t i = 0; i < n; i += kChunk) {
+    const int64_t m = std::min(n - i, kChunk);
+    N2W_CUDA(cudaMemcpy(cells.data(), b.d_seed + i, sizeof(int4) * static_cast<size_t>(m), cudaMemcpyDeviceToHost));
+    for (int64_t k = 0; k < m; ++k) out[i + k] = cells[static_cast<size_t>(k)].x;
+  }
 }
 
 void build_edges(n2w_bvh& b, int64_t triangles) {
