@@ -29,6 +29,7 @@ namespace {
 constexpr int kFrameBlock = 128;
 constexpr int kFrameMaxTris = 4096;
 constexpr int kFrameCandidates = 7;
+constexpr float kFrameFar = 1.0e30f;
 
 __device__ __forceinline__ float warp_min(float x) {
 #pragma unroll
@@ -104,7 +105,17 @@ __global__ void __launch_bounds__(kFrameBlock) frame_nodes_kernel(const Node4* _
     last[k] = c == kEmptyChild ? 0 : (c >= 0 ? ranges[c].last : leaf_first(c) + leaf_count(c));
   }
   float lo[4][3], hi[4][3];
-  const bool small = r.last - r.first <= kFrameMaxTris;
+  bool small = r.last - r.first <= kFrameMaxTris;
+  if (small) {
+    // a frame's arithmetic needs finite coordinates with finite squares
+    float far = 0.0f;
+    for (int k = 0; k < 4; ++k) {
+      if (nd.child[k] == kEmptyChild) continue;
+      far = fmaxf(far, fmaxf(fmaxf(fabsf(nd.lo_x[k]), fabsf(nd.hi_x[k])),
+                             fmaxf(fmaxf(fabsf(nd.lo_y[k]), fabsf(nd.hi_y[k])), fmaxf(fabsf(nd.lo_z[k]), fabsf(nd.hi_z[k])))));
+    }
+    small = far < 1.0e18f;
+  }
   if (small) {
     float nx = 0.0f, ny = 0.0f, nz = 0.0f, big = 0.0f;
     for (int t = r.first + lane; t < r.last; t += 32) {
@@ -156,8 +167,16 @@ __global__ void __launch_bounds__(kFrameBlock) frame_nodes_kernel(const Node4* _
   }
   // 2^-19 of the largest |vertex|_1: 8 u of the frame's rounding plus the
   // closest-point arithmetic's few u, twice over (u = 2^-24)
-  const float big1 = pad;
+  const float big1 = fminf(pad, kFrameFar);
   pad = pad * 1.9073486328125e-06f + 1e-30f;
+  // Planes end at kFrameFar, where a step's multiples are still finite; whatever lies
+  // beyond has no finite squared distance to any point that has one to anything.
+  for (int k = 0; k < 4; ++k) {
+    for (int a = 0; a < 3; ++a) {
+      lo[k][a] = fminf(fmaxf(lo[k][a] - pad, -kFrameFar), kFrameFar);
+      hi[k][a] = fminf(fmaxf(hi[k][a] + pad, -kFrameFar), kFrameFar);
+    }
+  }
   FrameNode4 o;
   o.vx = v.x;
   o.vy = v.y;
@@ -166,8 +185,8 @@ __global__ void __launch_bounds__(kFrameBlock) frame_nodes_kernel(const Node4* _
     float omin = INFINITY, omax = -INFINITY;
     for (int k = 0; k < 4; ++k) {
       if (nd.child[k] == kEmptyChild) continue;
-      omin = fminf(omin, lo[k][a] - pad);
-      omax = fmaxf(omax, hi[k][a] + pad);
+      omin = fminf(omin, lo[k][a]);
+      omax = fmaxf(omax, hi[k][a]);
     }
     // The step: a power of two with the children within 253 of them, at least
     // 2^-20 of the coordinates so the origin's rounding is a fraction of it.
@@ -183,8 +202,8 @@ __global__ void __launch_bounds__(kFrameBlock) frame_nodes_kernel(const Node4* _
     for (int k = 0; k < 4; ++k) {
       if (nd.child[k] == kEmptyChild) continue;
       // outwards by a quarter of a step, for the origin's and the quotient's rounding
-      const float bl = floorf((lo[k][a] - pad - origin) / step - 0.25f);
-      const float bh = ceilf((hi[k][a] + pad - origin) / step + 0.25f);
+      const float bl = floorf((lo[k][a] - origin) / step - 0.25f);
+      const float bh = ceilf((hi[k][a] - origin) / step + 0.25f);
       wl |= static_cast<uint32_t>(fminf(fmaxf(bl, 0.0f), 255.0f)) << (8 * k);
       wh |= static_cast<uint32_t>(fminf(fmaxf(bh, 0.0f), 255.0f)) << (8 * k);
     }
