@@ -527,7 +527,16 @@ void choose_nodes(n2w_bvh& b, int triangles, const dev::SeedGrid& grid) {
 // Where it reaches a quarter of the triangles' edge it covers patches of them, and the
 // axis-aligned boxes, which need none, leave far fewer to test: 81,920 triangles, work of
 // a query over frames / boxes 158 / 244 at 500 extents, 1,764 / 249 at 5,000.
-float far_limit(const n2w_bvh& b, const n2w_mesh& mesh) {
+float far_limit(const n2w_bvh& b, double edge) {
+  const double half = 0.5 * b.seed_n * static_cast<double>(b.seed_h);
+  double centre = 0.0;
+  for (int a = 0; a < 3; ++a) centre += std::fabs(b.seed_lo[a] + half);
+  const double far = (0.25 * edge - centre * 0x1p-20) / (5.3e-6 * half);
+  return static_cast<float>(far > 0.0 ? far : 0.0);  // (not a number: 0)
+}
+
+// Mean of the longer of two edges of each triangle.
+double mean_edge(const n2w_mesh& mesh) {
   double edge = 0.0;
   for (const auto& t : mesh.triangles) {
     double l2[2] = {0.0, 0.0};
@@ -538,12 +547,7 @@ float far_limit(const n2w_bvh& b, const n2w_mesh& mesh) {
     }
     edge += std::sqrt(std::max(l2[0], l2[1]));
   }
-  edge /= static_cast<double>(mesh.triangles.size());
-  const double half = 0.5 * b.seed_n * static_cast<double>(b.seed_h);
-  double centre = 0.0;
-  for (int a = 0; a < 3; ++a) centre += std::fabs(b.seed_lo[a] + half);
-  const double far = (0.25 * edge - centre * 0x1p-20) / (5.3e-6 * half);
-  return static_cast<float>(far > 0.0 ? far : 0.0);  // (not a number: 0)
+  return edge / static_cast<double>(mesh.triangles.size());
 }
 
 // Seed grid over the mesh box grown by 20 % of its largest extent on every side.
@@ -579,11 +583,15 @@ void build_seed_grid(n2w_bvh& b, const n2w_mesh& mesh, int n) {
     choose_nodes(b, static_cast<int>(mesh.triangles.size()),
                  dev::SeedGrid{coarse, b.seed_lo[0], b.seed_lo[1], b.seed_lo[2], 1.0f / (h * kSeedStride),
                                n / kSeedStride, INFINITY});
-    b.seed_far = far_limit(b, mesh);
+    const double edge = mean_edge(mesh);
+    b.seed_far = far_limit(b, edge);
     seed_grid_kernel<false><<<static_cast<unsigned>((total + block - 1) / block), block>>>(
         query_nodes_of(b), tris, b.seed_lo[0], b.seed_lo[1], b.seed_lo[2], h, n, coarse, b.d_seed, d_ov);
     N2W_CUDA(cudaGetLastError());
-    build_cell_entries(b);
+    // The cells' subtrees stand on computed distances being distances.  A triangle test
+    // multiplies four lengths: where that overflows or loses its digits a search starts at
+    // the root, as the cells say already.
+    if (edge > 1.0e-8 && static_cast<double>(h) * n < 1.0e9) build_cell_entries(b);
     N2W_CUDA(cudaMemcpy(&ov, d_ov, sizeof(int), cudaMemcpyDeviceToHost));
   } catch (...) {
     cudaFree(tmp);
