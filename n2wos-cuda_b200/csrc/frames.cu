@@ -218,8 +218,9 @@ __global__ void __launch_bounds__(kFrameBlock) frame_nodes_kernel(const Node4* _
 // cell, a cube of half-width `half` around the lattice node c, the closest
 // triangle is within D = d(c) + |x - c| <= d(c) + sqrt(3) half, so it lies in a
 // box only if the box is within D of the cube and within d(c) + 2 sqrt(3) half
-// of c.  Starting from the root, entries are replaced by their children that
-// pass both tests while they fit, so nothing that could be closest is left out.
+// of c, both widened by the rounding of d.  Starting from the root, entries are
+// replaced by their children that pass both tests while they fit, so nothing that could
+// be closest is left out.
 // Three subtrees: 18.0 -> 14.1 expansions per walk query (one: 16.2, two: 15.0;
 // more are visited in vain: eight 13.7 and 20 % more triangle tests), and the
 // cell stays one 16-byte load.
@@ -245,8 +246,22 @@ __global__ void __launch_bounds__(256) cell_entries_kernel(const float4* __restr
   const float scale = fabsf(c.x) + fabsf(c.y) + fabsf(c.z);
   const float half = 0.5005f * h + 4.0e-6f * scale, r = 1.7320509f * half;
   const float d = sqrtf(hit.d2);
-  const float lim_c = dev::prune_limit((d + 2.0f * r) * (d + 2.0f * r), c);
-  const float lim_q = dev::prune_limit((d + r) * (d + r), c);
+  // d(x) is a computed distance.  With edges up to L, height w over the longest and
+  // corners within D of x, the test's dot products are off by 5 u L D, its barycentric
+  // numerators by 23 u (L D)^2, its denominator (L w)^2 by three times that, so the point by
+  // 115 u D^2 / w^2 of L, here and at the lattice node.  Where that is no longer small (a
+  // sliver, whose test may even divide by zero) the cell keeps the root.
+  const dev::Rec64 t = dev::load_rec<false>(tris, slot);
+  const dev::V3 ab = dev::v3(t.r1.x, t.r1.y, t.r1.z), ac = dev::v3(t.r1.w, t.r2.x, t.r2.y),
+                bc = dev::vsub(ac, ab);
+  const dev::V3 nrm = dev::v3(ab.y * ac.z - ab.z * ac.y, ab.z * ac.x - ab.x * ac.z, ab.x * ac.y - ab.y * ac.x);
+  const float edge2 = fmaxf(dev::vdot(ab, ab), fmaxf(dev::vdot(ac, ac), dev::vdot(bc, bc)));
+  const float height2 = dev::vdot(nrm, nrm) / edge2, corner = d + 2.0f * r + sqrtf(edge2);
+  const float off = 1.52587890625e-05f * corner * corner / height2;  // 2 x 128 u
+  if (!(off < 0.25f)) return;
+  const float reach = d + r + off * sqrtf(edge2);
+  const float lim_c = dev::prune_limit((reach + r) * (reach + r), c);
+  const float lim_q = dev::prune_limit(reach * reach, c);
   int e[dev::kCellEntries] = {0, kEmptyChild, kEmptyChild};
   int count = 1;
   if (hit.id != INT32_MAX) {
