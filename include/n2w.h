@@ -594,7 +594,8 @@ typedef struct n2w_batch_item {
 typedef struct n2w_batch_tuning {
   int32_t block_size;      /* walker threads per block: 64, 128 or 256 */
   int32_t blocks_per_sm;   /* 0 = occupancy maximum */
-  int32_t chunk;           /* walks a lane takes per queue pop */
+  int32_t chunk;           /* most walks a lane takes per queue pop (fewer while its share of the launch
+                              is below 64 times that) */
   int32_t regen_threshold; /* waiting lanes that trigger walk updates */
   int32_t reg_variant;     /* 0: 64 registers / 4 blocks per SM; 1: 80 registers / 3 blocks */
   float ms;                /* autotuner: best time of this shape on the probe batch */

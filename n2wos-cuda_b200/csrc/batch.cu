@@ -37,6 +37,7 @@ struct n2w_batch {
   const n2w_scene* scene = nullptr;
   int n_items = 0;
   int64_t total_points = 0, total_chunks = 0;
+  int chunk = 1;  // walks per queue pop of this launch (launch_chunk)
   n2w_walk_options opt{};
   int reg_variant = 0;
   std::vector<n2w_batch_item> items;
@@ -98,9 +99,21 @@ __global__ void zero_batch_stats_kernel(const BatchInst* __restrict__ insts, int
   I.forced[q] = 0u;
 }
 
-// Smallest chunk the autotuner offers (its results are documented as 2, 4, 8 or
-// 16); against single-walk chunks it costs 1 % (44.0 -> 44.5 ms, 48 instances).
+// Smallest chunk the autotuner offers, as the options' largest: see launch_chunk.
 constexpr int kTunedChunkMin = 2;
+
+// Walks a lane takes per queue pop: the options' number (the autotuner's 2, 4, 8 or 16,
+// or 1) at most, and no more than a 64th of a lane's share of the launch.  A launch ends
+// with its slowest lane's last chunk, a serial chain of that many walks; chunk 1 / 2 / 8:
+// 2.2 / 3.1 / 8.1 ms for 5,575 walks in 8 instances, 3.4 / 4.6 / 8.5 for 62,780 in 48,
+// 32.7 / 33.8 / 40.4 for 5.0 M.  At hundreds of walks per lane they are equal.
+int launch_chunk(const n2w_batch& b) {
+  int64_t walks = 0;
+  for (const auto& it : b.items) walks += it.point_count * it.walks_per_point;
+  const int64_t lanes = static_cast<int64_t>(sm_count_current()) * kWalkerMinBlocks * kDefaultWalkerThreads;
+  const int64_t most = b.opt.chunk > 0 ? b.opt.chunk : kDefaultChunk;
+  return static_cast<int>(std::max<int64_t>(std::min(walks / (64 * lanes), most), 1));
+}
 
 unsigned blocks_of(int64_t n, int b) { return static_cast<unsigned>((n + b - 1) / b); }
 
@@ -114,7 +127,7 @@ void free_graph(n2w_batch& b) {
 // Builds the instance table (host) from the items and current options.
 void build_instances(n2w_batch& b) {
   const n2w_scene& sc = *b.scene;
-  const int chunk = b.opt.chunk > 0 ? b.opt.chunk : kDefaultChunk;
+  const int chunk = b.chunk = launch_chunk(b);
   b.h_insts.assign(b.n_items, BatchInst{});
   int64_t pbase = 0, cbase = 0;
   for (int k = 0; k < b.n_items; ++k) {
@@ -157,7 +170,7 @@ WalkArgs batch_args(const n2w_batch& b, n2w_walk_counters* d_counters) {
   a.first_cpd = b.d_cpd;
   a.first_ids = b.d_ids;
   a.total_chunks = b.total_chunks;
-  a.chunk = b.opt.chunk > 0 ? b.opt.chunk : kDefaultChunk;
+  a.chunk = b.chunk;
   a.regen = b.opt.regen_threshold > 0 ? b.opt.regen_threshold : kDefaultRegen;
   a.max_steps = b.opt.max_steps;
   a.eps = b.opt.epsilon;

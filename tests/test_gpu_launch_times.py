@@ -83,3 +83,20 @@ def test_few_walks_share_the_warps_that_the_caller_leaves(gpu, small_and_large):
     limited, free = timed_in_turn(gpu, [walk_call(gpu, small_and_large[1], pts, walks_per_point=16, **o) for o in
                                         (dict(blocks_per_sm=1, block_size=32), {})])
     assert limited < 2.0 * free, (limited, free)
+
+
+def test_chunks_do_not_slow_small_batches(gpu, small_and_large):
+    """A batch of few walks with the autotuner's smallest and largest chunks, and autotuned, against the batch as
+    created: the chunk is a limit, and a lane's share of this launch is below one walk."""
+    scene = gpu.Scene([small_and_large[1]])
+    rng = np.random.default_rng(6)
+    inst = [{"mesh": 0, "problem": 0, "points": rng.uniform(-0.3, 0.3, (100, 3)).astype(np.float32),
+             "walks_per_point": 24, "seed": 40 + i} for i in range(4)]
+    problems = [gpu.problem_charges_seeded(8, 1.6, 2.0, 3)]
+    batches = [gpu.Batch(scene, problems, inst, gpu.walk_options(epsilon=1e-3)) for _ in range(4)]
+    shape = {"block_size": 128, "blocks_per_sm": 0, "regen_threshold": 16, "reg_variant": batches[0].info()["reg_variant"]}
+    batches[1].set_tuning({**shape, "chunk": 2})
+    batches[2].set_tuning({**shape, "chunk": 16})
+    batches[3].autotune(1.0)
+    plain, two, sixteen, tuned = timed_in_turn(gpu, [lambda s, b=b: b.launch(s) for b in batches])
+    assert max(two, sixteen, tuned) < 1.2 * plain, (plain, two, sixteen, tuned)
