@@ -3,7 +3,8 @@
 // variant, src/cuda/cubql_bvh.cu:187-214).  Each query is seeded with the
 // triangle stored at the nearest seed-grid node (a real candidate, so the
 // exact answer is unchanged), started at that cell's subtrees and finished by
-// the search over the frame nodes of geom.cuh, or by a whole warp
+// the search over the frame nodes of geom.cuh, or over the axis-aligned ones
+// where those are the better (choose_nodes, far_limit), or by a whole warp
 // (warp_search.cuh).
 #include <cuda_runtime.h>
 
@@ -62,7 +63,7 @@ constexpr int kQueryBlock = 256;
 // surface), 170 / 153 / 158 / 151 / 151 us (40,000); 4,194,304: the same.
 constexpr uint32_t kQueryBudget = 112;
 constexpr uint32_t kBoxBudget = 384;  // the same over the boxes, whose long queries have more nodes to visit
-constexpr int kFinishWarps = 32;    // resident warps per SM of the finisher (62 registers, 4 KiB each)
+constexpr int kFinishWarps = 32;    // warps per SM that a finisher launch aims at (24 are resident: 78 registers)
 constexpr int kHandOff = 2;         // overflow-slot mark of a handed-off query
 constexpr int kHandOffFar = 3;      // the same for a far one (far_limit), handed off as soon as it is seeded
 // Between warp_query_limit and kShortQueries a lane keeps only the queries whose seed lies
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) closest_point_finish
     int4 start = make_int4(0, 0, kEmptyChild, kEmptyChild);  // the root
     bool at_far;
     if (grid.cells) start = dev::seed_cell_any(grid, p, 0, at_far);
-    dev::warp_search(nodes, tris, p, start, (far >> i) & 1u, b, work);
+    dev::warp_search<false>(nodes, tris, p, start, (far >> i) & 1u, b, work);
     if (b.winner()) {
       const int id = static_cast<int>(b.key & 0xffffffffu);
       out_d2[q] = dev::key_d2(b.key);
@@ -249,8 +250,13 @@ __global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) closest_point_finish
   }
 }
 
-// Small launches: one warp per query (warp_search.cuh).
-template <bool kMasked>
+// Small launches: one warp per query (warp_search.cuh).  The smallest are as short as the
+// code they fetch and run without the search over boxes: 1,000 / 40 queries of 5,120
+// triangles, waited for, 16.9 / 14.9 -> 15.9 / 14.3 us.  (1,000 queries 50,000 extents from
+// 81,920 triangles then take 1.1 ms instead of 0.04; 5,000 extents 0.2.)
+constexpr int kFramesOnlyQueries = 2048;
+
+template <bool kMasked, bool kFramesOnly>
 __global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) closest_point_warp_kernel(
     const dev::QueryNodes nodes, const float4* __restrict__ tris, const dev::SeedGrid grid,
     const n2w_vec3* __restrict__ points, const uint8_t* __restrict__ active, int n, float* __restrict__ out_d2,
@@ -269,8 +275,8 @@ __global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) closest_point_warp_k
     }
     return;
   }
-  const dev::WarpBest b = dev::warp_query(nodes, tris, grid, dev::v3(pt.x, pt.y, pt.z), 0, dev::v3(0.0f, 0.0f, 0.0f),
-                                          s_work + warp * dev::kWarpList);
+  const dev::WarpBest b = dev::warp_query<kFramesOnly>(nodes, tris, grid, dev::v3(pt.x, pt.y, pt.z), 0,
+                                                       dev::v3(0.0f, 0.0f, 0.0f), s_work + warp * dev::kWarpList);
   if (b.winner()) {
     const int id = static_cast<int>(b.key & 0xffffffffu);
     out_d2[q] = dev::key_d2(b.key);
@@ -455,7 +461,9 @@ void launch_closest_point(const n2w_bvh& bvh, const n2w_vec3* d_points, const ui
   }
   if (n <= warp_query_limit(bvh.stats.triangles, nodes.use_boxes, false)) {
     const unsigned blocks = static_cast<unsigned>((n + dev::kWarpsPerBlock - 1) / dev::kWarpsPerBlock);
-    auto kern = d_active ? closest_point_warp_kernel<true> : closest_point_warp_kernel<false>;
+    const bool frames_only = n <= kFramesOnlyQueries && !nodes.use_boxes;
+    auto kern = d_active ? (frames_only ? closest_point_warp_kernel<true, true> : closest_point_warp_kernel<true, false>)
+                         : (frames_only ? closest_point_warp_kernel<false, true> : closest_point_warp_kernel<false, false>);
     kern<<<blocks, 32 * dev::kWarpsPerBlock, dev::kWarpSearchBytes, stream>>>(nodes, tris, sg, d_points, d_active, n,
                                                                              d_d2, d_cp, d_id, d_overflow);
     N2W_CUDA(cudaGetLastError());

@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(32 * dev::kWarpsPerBlock) first_query_warp_ker
   if (i >= n) return;
   const FirstQuery f = first_query_of<kBatch>(a, i);
   const dev::WarpBest b =
-      dev::warp_query(dev::QueryNodes{a.nodes, a.boxes, a.first_boxes != 0}, a.tris, f.grid, f.p, f.root, f.p,
+      dev::warp_query<false>(dev::QueryNodes{a.nodes, a.boxes, a.first_boxes != 0}, a.tris, f.grid, f.p, f.root, f.p,
                       s_work + warp * dev::kWarpList);
   if (b.winner()) {
     cpd[i] = make_float4(b.cp.x, b.cp.y, b.cp.z, dev::key_d2(b.key));

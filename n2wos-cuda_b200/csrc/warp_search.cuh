@@ -63,7 +63,7 @@ __device__ __forceinline__ void warp_search_over(const float4* __restrict__ node
   int sp = 3;  // warp-uniform
   __syncwarp();
   while (sp > 0) {
-    const int take = min(min(sp, 32), max((kWarpList - kWarpReserve - sp) / 3, 1));  // sp + 3 take spares the reserve
+    const int take = min(min(sp, 32), max((kWarpList - kWarpReserve - sp) >> 2, 1));  // sp + 3 take spares the reserve
     int2 e = make_int2(kEmptyChild, 0);
     if (lane < take) e = work[sp - take + lane];
     __syncwarp();
@@ -137,13 +137,16 @@ __device__ __forceinline__ void warp_search_over(const float4* __restrict__ node
   }
 }
 
+template <bool kFramesOnly>
 __device__ __forceinline__ void warp_search(const QueryNodes& nodes, const float4* __restrict__ tris, V3 p, int4 start,
                                             bool far, WarpBest& b, int2* work) {
-  if (nodes.use_boxes || far) warp_search_over<true>(nodes.boxes, tris, p, start, b, work);
+  if (!kFramesOnly && (nodes.use_boxes || far)) warp_search_over<true>(nodes.boxes, tris, p, start, b, work);
   else warp_search_over<false>(nodes.frames, tris, p, start, b, work);
 }
 
-// A cold query, seeded and started by the grid if there is one.
+// A cold query, seeded and started by the grid if there is one.  kFramesOnly: without the
+// search over boxes, for trees over frames, far points included.
+template <bool kFramesOnly>
 __device__ __forceinline__ WarpBest warp_query(const QueryNodes& nodes, const float4* __restrict__ tris,
                                                const SeedGrid& grid, V3 p, int root, V3 no_hit, int2* work) {
   ClosestHit h;
@@ -154,14 +157,14 @@ __device__ __forceinline__ WarpBest warp_query(const QueryNodes& nodes, const fl
   int4 cell = make_int4(0, root, kEmptyChild, kEmptyChild);
   bool far = false;
   if (grid.cells) {
-    cell = nodes.seed(grid, p, root, far);
+    cell = kFramesOnly ? seed_cell_any(grid, p, root, far) : nodes.seed(grid, p, root, far);
     test_slot(tris, cell.x, p, h);
   }
   WarpBest b;
   b.key = b.mine = hit_key(h.d2, h.id);
   b.cp = h.cp;
   b.slot = h.slot;
-  warp_search(nodes, tris, p, cell, far, b, work);
+  warp_search<kFramesOnly>(nodes, tris, p, cell, far, b, work);
   if (grid.cells && (threadIdx.x & 31) == 0) ++b.tris;
   return b;
 }
